@@ -27,13 +27,13 @@
 //              cancel are skipped as d3 skips them), FP64 centroid sums for the top levels.
 //   slots      each cell writes its children (position or centroid, value at own depth, and for
 //              a child cell its child range and depth) into its slots
-//   walk       a group of G consecutive sorted points (G = 32: a warp, or 16) walks the union of
-//              their d3 traversals: batches of up to G children are gathered from the group's
-//              stack in shared memory and loaded lane-parallel, and every lane applies apply()
-//              of manyBody.js for its own point, two children per round in packed FP32 pairs:
-//              a cell is approximated at the first (widest) depth of its chain where
+//   walk       a warp walks the union of the d3 traversals of 32 (or 16) consecutive sorted
+//              points: rounds of up to 32 children are gathered from the group's stack in shared
+//              memory, classified lane-parallel against the group's bounding box, and every lane
+//              applies apply() of manyBody.js for its own point, two children per step in packed
+//              FP32 pairs: a cell is approximated at the first (widest) depth of its chain where
 //              w^2 / theta^2 < l, points are summed exactly, distanceMin / distanceMax as d3;
-//              cells that some lane must open are pushed with the mask of those lanes.
+//              cells that some point must open are pushed with the mask of those points.
 //
 // Points with the same code at the finest level share the deepest cell as its children.
 #include <math.h>
@@ -929,11 +929,14 @@ __global__ void __launch_bounds__(kThreads) k_slots(
 constexpr int kWalkThreads = 128;
 constexpr int kWalkWarps = kWalkThreads / 32;
 constexpr int kStack = 96;  // entries per group in shared memory; deeper entries spill to global
-// A group's stack never holds more than (levels + 1) * G entries: every batch pushes at most G
-// entries (the cells its lanes open), and the entries on the stack form layers, one per batch
+// A group's stack never holds more than (levels + 1) * 32 entries: every round pushes at most 32
+// entries (the cells its points open), and the entries on the stack form layers, one per round
 // whose pushes are not yet consumed, holding cells of strictly increasing depth.
 __host__ __device__ constexpr int kWalkStackLayers(int ndim) { return (ndim == 3 ? 21 : 24) + 1; }
-constexpr int kWalkSpillPerWarp = 704;  // max over dims and group sizes of NG ((levels+1) G - kStack)
+constexpr int kWalkSpillPerWarp = 704;  // max over dims of 32 (levels + 1) - kStack
+// Blocks per SM the walk's registers are held to: at 1M nodes 8 (64 registers) measured 740 us a
+// launch, 9 (56) 746, 7 (72) 766.
+constexpr int kWalkMinBlocks = 8;
 constexpr int kWalkBlocksPerSm = 10;    // blocks of the persistent walk grid per SM
 // the largest layout whose walk runs one point per warp by default (FL_TUNE_WALK_GROUP 0)
 constexpr int kLaneWalkMaxNodes = 32768;
@@ -970,17 +973,18 @@ __device__ __forceinline__ float rcp_approx(float x) {  // the reciprocal __fdiv
   return r;
 }
 
-template <int NG>
+constexpr int kSeenWords = 64;  // a group's coordinate filter: 2,048 bits per axis
+// A warp's walk state. The round's children are kept as pairs (2j, 2j + 1) in the packed layout
+// that the f32x2 arithmetic reads.
 struct WalkShared {
-  uint4 stack[kWalkWarps][NG][kStack];  // per point group: first child slot, count, top depth, lanes
-  // the batches, one entry per child: what every test reads ...
-  // per pair of children (2j, 2j + 1): {x, x', y, y'} and {z, z', value, value'}, the value at
-  // the chain's top depth times alpha, in the packed layout the f32x2 arithmetic reads
-  float4 data[kWalkWarps][32];
-  uint4 test[kWalkWarps][32];   // open threshold, uncommon-case bound, lane mask, slot / index
-  // ... and what only a push or an uncommon case reads
-  uint2 cold[kWalkWarps][32];   // meta word (count | depth << 26, or kLeafMark), chain top depth
-  uint32_t own[kWalkWarps][32];  // the gather: which stack entry each child of the batch is from
+  uint4 stack[kStack];  // first child slot, count, top depth, the points that test the children
+  float4 a[16];         // {x, x', y, y'}
+  float4 b[16];         // {z, z', value, value'}: at the chain's top depth, times alpha
+  float4 t[16];         // {theta threshold, ', uncommon cases' bound, '}
+  uint32_t mask[32];    // the points that test each child
+  uint32_t opens[32];   // the points that open each child
+  uint32_t seen[3][kSeenWords];
+  float4 lo, hi;        // the group's bounding box
 };
 
 // The less common cases of apply() (src/manyBody.js:73-115) for one child: a chain of cells
@@ -1019,285 +1023,346 @@ __device__ __forceinline__ void rare_case(uint32_t meta, uint32_t top, uint32_t 
   if (l < dmin2) l = sqrtf(dmin2 * l);
 }
 
-// The walk of G consecutive sorted points (G = 32: a warp; 16: half a warp each, with its own
-// stack and batches, so that fewer points share, and pay for, one union of traversals).
-//
-// Per child and testing lane, the common case costs one theta compare (opened?), one compare
-// against the uncommon-case bound, the force and two ballots. The bound folds two tests into
-// one: a chain cell whose widest depth is too close for this point (l <= threshold at the top
-// depth) and distanceMin (l < dmin2, i.e. l <= the float below dmin2).
-// stats (STATS): [0] child tests (G per child), [1] tests a lane's own traversal needed,
-// [2] deepest stack, [3] lanes that opened a cell, [4] lanes that applied a cell or point,
-// [5] pair rounds that took the uncommon-case branch.
 __device__ __forceinline__ float below(float d2) {  // l < d2 <=> l <= below(d2), for l >= 0
   return d2 > 0.f ? __uint_as_float(__float_as_uint(d2) - 1u) : -1.f;
 }
+// 1 << i, 0 for i >= 32.
+__device__ __forceinline__ uint32_t bit_at(uint32_t i) {
+  uint32_t r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(i));
+  return r;
+}
+// The warp's inclusive prefix sum (shfl.up's predicate says whether the lane below exists).
+__device__ __forceinline__ uint32_t inclusive_sum(uint32_t v) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .u32 t;\n\t"
+        "shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t"
+        "@p add.u32 %0, %0, t;\n\t}"
+        : "+r"(v) : "r"(o));
+  return v;
+}
+// A coordinate's bit of the filter (a multiplicative hash, 2^32 / golden ratio times 2): the sign
+// is left out, so that 0 and -0 share a bit.
+__device__ __forceinline__ uint32_t seen_bit(float x) {
+  return (__float_as_uint(x) * 0x3c6ef362u) >> 21;
+}
+__device__ __forceinline__ bool maybe_seen(const uint32_t* seen, float x) {
+  const uint32_t h = seen_bit(x);
+  return seen[h >> 5] >> (h & 31u) & 1u;
+}
 
-// BATCH: the points belong to a batch of graphs (segs): each graph has its own tree (root slot =
-// its index), cube, theta, distances and alpha; a group's points may span graphs.
-template <int NDIM, int G, bool STATS, bool DMAX, bool BATCH>
-__global__ void __launch_bounds__(kWalkThreads) k_walk(
+// The walk of P consecutive sorted points by a warp: P = 32, a point per lane, or P = 16, two
+// lanes per point that take every other pair of children (fewer points share, and pay for, one
+// union of traversals).
+//
+// Per round the warp gathers 32 children, one per lane, and each lane decides from the group's
+// bounding box what its child can need. The displacement, its square and their sum round
+// monotonically, so the box's nearest squared distance bounds every point's own:
+//   far    no point opens it and none takes an uncommon case: it is only applied
+//   plain  some points may open it, but none takes an uncommon case
+//   odd    distanceMin, a chain's widest cell or a coordinate that one of the points may share (a
+//          zero component, which d3 jiggles) can occur
+// A shared coordinate is looked for in a filter of the group's coordinates, 2,048 bits per axis,
+// and only where the child lies within the box on that axis. Then every lane takes the children
+// in order, two per step, with the tests that the pair's classes ask for: the same FP32 sums, in
+// the same order, as testing every pair for everything.
+//
+// The pass is bound by instruction issue (79 % of the issue slots). At 1M nodes in 3D a group meets
+// 687 children in 24.4 rounds, of which a point's own traversal needs 43 %; 61 % are far, 22 %
+// plain. Measured with events, testing every pair for everything -> this: 791 -> 740 us a launch
+// (1M nodes, 3D), 292 -> 259 (300k, distanceMax), 99 -> 92 (200k, 2D), 117 -> 113 (100k, 3D). Two
+// far steps at once, not one (765 us) nor four (777). Applying the far children later, 32 at a
+// time without tests, took 613 us, but adds each point's terms in another order.
+//
+// stats (STATS): [0] child tests (P per child), [1] tests a point's own traversal needed,
+// [2] deepest stack, [3] points that opened a cell, [4] points that applied a cell or point,
+// [5] pair steps that took the uncommon-case branch.
+// BATCH: the points belong to a batch of graphs (segs): a group is up to 32 points of one graph,
+// with its tree (root slot = its index), cube, theta, distances and alpha.
+template <int NDIM, int P, bool STATS, bool DMAX, bool BATCH>
+__global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks) k_walk(
     const float4* __restrict__ cdata, const uint2* __restrict__ cmeta,
     const float4* __restrict__ leaf, const uint32_t* __restrict__ perm,
     const float* __restrict__ cube, float4* __restrict__ vel, int n, float alpha,
     double theta2, float dmin2, float dmax2, uint32_t step, uint32_t seed, uint32_t* err,
-    unsigned long long* stats, uint4* __restrict__ spill, int nwarps, uint32_t* work,
+    unsigned long long* stats, uint4* __restrict__ spill, int ngroups, uint32_t* work,
     FlSegs segs, const FlTick* __restrict__ tk) {
   if (tk) alpha = tk->alpha, step = tk->step, seed = tk->seed;
-  constexpr int NG = 32 / G;
-  // the stack of a group: kStack entries in shared memory, then up to kWalkStack(NDIM, G) in
-  // all, the rest in this warp slot's region of the spill buffer
-  constexpr int kAll = kWalkStackLayers(NDIM) * G, kSpilled = kAll - kStack;
-  static_assert(NG * kSpilled <= kWalkSpillPerWarp, "spill region too small");
-  __shared__ WalkShared<NG> sh;
+  constexpr int S = 32 / P;  // lanes per point
+  constexpr uint32_t kPoints = P == 32 ? FL_FULL : (1u << (P & 31)) - 1u;
+  // the stack: kStack entries in shared memory, the rest in this warp slot's region of the spill
+  // buffer (at most 32 pushes a round, layers of strictly increasing depth)
+  constexpr int kAll = kWalkStackLayers(NDIM) * 32;
+  static_assert(kAll - kStack <= kWalkSpillPerWarp, "spill region too small");
+  __shared__ WalkShared shw[kWalkWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = lane / G, gl = lane % G, gbase = grp * G;
-  const uint32_t gmask = G == 32 ? FL_FULL : (((1u << G) - 1u) << gbase);
-  const uint32_t lanebit = 1u << lane;
+  WalkShared& sh = shw[warp];
+  const int sub = lane / P;
+  const uint32_t lanebit = 1u << (lane % P), below_me = (1u << lane) - 1u;
   // (size / 2^k)^2 / theta^2 = T0 * 4^-k, exactly (a power-of-two scaling); the FP64 division
   // once per block
   __shared__ float s_T0;
   if (!BATCH && threadIdx.x == 0) s_T0 = (float)((double)cube[3] * (double)cube[3] / theta2);
   __syncthreads();
-  const float T0 = BATCH ? 0.f : s_T0;
-  // l < dmin2  <=>  l <= the largest float below dmin2 (l >= 0)
-  const float dmin_le = below(dmin2);
+  float T0 = BATCH ? 0.f : s_T0;
+  uint32_t gfirst = 0, gstep = step, gcount = (uint32_t)n, gcells = 0;
   const uint32_t slot_cap = 2u * (uint32_t)n + 1u;
   unsigned long long st_tests = 0, st_useful = 0, st_open = 0, st_apply = 0, st_rare = 0;
   int maxsp = 0;
-  const int wslot = blockIdx.x * kWalkWarps + warp;  // this warp's slot of a persistent grid
-  uint4* stk = sh.stack[warp][grp];
-  uint4* spl = spill + (size_t)wslot * kWalkSpillPerWarp + grp * kSpilled;
-  auto sget = [&](int i) { return i < kStack ? stk[i] : spl[i - kStack]; };
+  uint4* spl = spill + (size_t)(blockIdx.x * kWalkWarps + warp) * kWalkSpillPerWarp;
+  auto sget = [&](int i) { return i < kStack ? sh.stack[i] : spl[i - kStack]; };
   auto sset = [&](int i, uint4 v) {
-    if (i < kStack) stk[i] = v;
+    if (i < kStack) sh.stack[i] = v;
     else spl[i - kStack] = v;
   };
-  float4* spair = sh.data[warp] + gbase;
-  uint4* stest = sh.test[warp] + gbase;
-  uint2* scold = sh.cold[warp] + gbase;
-  // groups of 32 points are handed out one at a time (the walk's cost varies a lot between
-  // groups, so a fixed share per warp would leave some warps working long after the rest)
+  // groups are handed out one at a time (the walk's cost varies a lot between groups, so a fixed
+  // share per warp would leave some warps working long after the rest)
   int wi = lane == 0 ? (int)atomicAdd(work, 1u) : 0;
   wi = __shfl_sync(FL_FULL, wi, 0);
-  while (wi < nwarps) {
-  // a group: 32 consecutive sorted points, or in a batch one graph's points [x, y), at most 32
-  const uint2 grp_range = BATCH ? segs.groups[wi] : make_uint2((uint32_t)wi * 32u, (uint32_t)n);
-  const int base = (int)grp_range.x;
-  const int t = base + lane;
-  const bool live = t < (int)grp_range.y;
-  const uint32_t act = __ballot_sync(FL_FULL, live) & gmask;
-  const float4 me = live ? leaf[t] : make_float4(0, 0, 0, 0);
-  const uint32_t myid = live ? perm[t] : 0;
-  uint64_t AX = 0, AY = 0, AZ = 0;  // force sums, one per child of a round's pair
-  const uint64_t MX = pk2(me.x, me.x), MY = pk2(me.y, me.y), MZ = pk2(me.z, me.z);
-  // the lane's own graph: what its uncommon cases and distanceMax use
-  float myT0 = T0, mydmin2 = dmin2, mydmax2 = dmax2;
-  uint32_t myfirst = 0, mystep = step, myng = (uint32_t)n, mycb = 0;
-  int sp;
-  if (!BATCH) {
-    if (gl == 0 && act) sset(0, make_uint4(0u, 1u, 0u, act));  // the root: slot 0, top depth 0
-    sp = act ? 1 : 0;
-  } else {
-    // one root entry per graph among the group's points (a graph of one point has no tree);
-    // a stack entry's third word is its top depth | graph << 8
-    const uint32_t g = live ? segs.gid_pos[t] : 0xffffffffu;
-    bool tree = false;
-    if (live) {
+  while (wi < ngroups) {
+    const uint2 range = BATCH ? segs.groups[wi]
+                              : make_uint2((uint32_t)wi * P, min((uint32_t)wi * P + P, (uint32_t)n));
+    const int base = (int)range.x;
+    const int t = base + lane % P;
+    const bool live = t < (int)range.y;
+    const uint32_t act = __ballot_sync(FL_FULL, live) & kPoints;
+    const float4 me = live ? leaf[t] : make_float4(0, 0, 0, 0);
+    const uint32_t myid = live ? perm[t] : 0;
+    uint4 root = make_uint4(0u, 1u, 0u, act);  // slot 0, one child, top depth 0
+    int sp = 1;
+    if (BATCH) {
+      const uint32_t g = segs.gid_pos[base];
       const FlGraph& gr = segs.g[g];
-      myT0 = gr.T0, mydmin2 = gr.dmin2, mydmax2 = gr.dmax2;
-      myfirst = (uint32_t)gr.first, mystep = step + gr.tick0, myng = (uint32_t)gr.count;
+      T0 = gr.T0, dmin2 = gr.dmin2, dmax2 = gr.dmax2, alpha = gr.alpha;
+      gfirst = (uint32_t)gr.first, gstep = step + gr.tick0, gcount = (uint32_t)gr.count;
+      root.x = g;
       // the graph's root sits in slot g; its first child slot less one is where the graph's
       // slots are counted from (a lone simulation's root has its children from slot 1)
-      if (gr.count > 1) mycb = __ldg(&cmeta[g].x) - 1u;
-      tree = gr.count > 1 && !gr.frozen;
+      if (gr.count > 1) gcells = __ldg(&cmeta[g].x) - 1u;
+      if (gr.count < 2 || gr.frozen) sp = 0;  // no tree, or sitting the tick out
     }
-    const uint32_t peers = __match_any_sync(FL_FULL, tree ? g : 0xffffffffu) & gmask;
-    const bool leader = tree && (peers & (lanebit - 1u)) == 0;
-    const uint32_t leaders = __ballot_sync(FL_FULL, leader) & gmask;
-    if (leader) sset(__popc(leaders & (lanebit - 1u)), make_uint4(g, 1u, g << 8, peers));
-    sp = __popc(leaders);
-  }
-  if (sp > maxsp) maxsp = sp;
-  __syncwarp();
-  uint32_t guard = 0;
-  const uint32_t guard_max = 4u * (uint32_t)n + 64u;
-  while (__any_sync(FL_FULL, sp > 0)) {
-    // each group gathers the first G children from the top of its stack, in parallel: lane gl
-    // reads the gl-th entry from the top, a prefix sum of the entries' child counts places each
-    // entry's children in the batch, and lane gl then finds the entry of the batch's gl-th child
-    const bool has = gl < sp;
-    uint4 e = has ? sget(sp - 1 - gl) : make_uint4(0u, 0u, 0u, 0u);
-    if (has && (e.x >= slot_cap || e.y > slot_cap - e.x)) {  // a malformed tree: never read past it
-      atomicOr(err, FL_ERR_TREE);
-      e.y = e.x >= slot_cap ? 0u : slot_cap - e.x;
-    }
-    uint32_t inc = e.y;
+    const float dmin_le = below(dmin2);
+    // the group's box and coordinate filter
+    for (int i = lane; i < 3 * kSeenWords; i += 32) (&sh.seen[0][0])[i] = 0u;
+    {
+      const float c[3] = {me.x, me.y, me.z};
+      float blo[3] = {0.f, 0.f, 0.f}, bhi[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(FL_FULL, inc, o, G);
-      if (gl >= o) inc += u;
-    }
-    const uint32_t exc = inc - e.y;
-    const uint32_t avail = __shfl_sync(FL_FULL, inc, G - 1, G);
-    const int total = avail < (uint32_t)G ? (int)avail : G;
-    // entries taken whole leave the stack; one taken in part keeps the rest (the new top)
-    const uint32_t taken = __ballot_sync(FL_FULL, has && inc <= (uint32_t)total) & gmask;
-    if (has && exc < (uint32_t)total && inc > (uint32_t)total)
-      sset(sp - 1 - gl, make_uint4(e.x + ((uint32_t)total - exc), inc - (uint32_t)total, e.z, e.w));
-    sp -= __popc(taken);
-    // each entry marks where its children start; a running max carries the mark to the rest
-    uint32_t* sown = sh.own[warp] + gbase;
-    sown[gl] = 0u;
-    __syncwarp();
-    if (e.y && exc < (uint32_t)total) sown[exc] = (uint32_t)gl;
-    __syncwarp();
-    uint32_t own = sown[gl];
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(FL_FULL, own, o, G);
-      if (gl >= o && u > own) own = u;
-    }
-    const uint32_t own_first = __shfl_sync(FL_FULL, e.x, (int)own, G);
-    const uint32_t own_exc = __shfl_sync(FL_FULL, exc, (int)own, G);
-    const uint32_t my_mask = __shfl_sync(FL_FULL, e.w, (int)own, G);
-    const uint32_t my_z = __shfl_sync(FL_FULL, e.z, (int)own, G);
-    const uint32_t my_top = my_z & 0xffu, my_g = my_z >> 8;
-    const uint32_t my_slot = own_first + ((uint32_t)gl - own_exc);
-    __syncwarp();
-    const int jmax = G == 32 ? total : (int)__reduce_max_sync(FL_FULL, (unsigned)total);
-    if (gl < total) {
-      // what does not depend on the testing point, once per child
-      const float4 q = __ldg(cdata + my_slot);
-      const uint2 m = __ldg(cmeta + my_slot);
-      const bool lf = m.y == kLeafMark;
-      const uint32_t D = (m.y >> 26) & 31u;
-      uint32_t mask = q.w != 0.f ? my_mask : 0u;  // d3 skips a zero value and all it holds
-      if (lf && m.x - (uint32_t)base < 32u) mask &= ~(1u << (m.x - (uint32_t)base));  // itself
-      const bool chain = !lf && my_top < D;
-      float T0c = T0, alc = alpha, dminc = dmin_le;
-      if (BATCH) {  // the child's graph: that of the lanes that test it
-        const FlGraph& gr = segs.g[my_g];
-        T0c = gr.T0, alc = gr.alpha, dminc = below(gr.dmin2);
+      for (int k = 0; k < NDIM; ++k) {
+        // a NaN coordinate bounds nothing: its tests all fail, whatever the child's class
+        const bool in = live && c[k] == c[k];
+        blo[k] = fl::unordered(__reduce_min_sync(FL_FULL, in ? fl::ordered(c[k]) : 0xffffffffu));
+        bhi[k] = fl::unordered(__reduce_max_sync(FL_FULL, in ? fl::ordered(c[k]) : 0u));
       }
+      if (lane == 0) {
+        sh.lo = make_float4(blo[0], blo[1], blo[2], 0.f);
+        sh.hi = make_float4(bhi[0], bhi[1], bhi[2], 0.f);
+        sset(0, root);
+      }
+      __syncwarp();
+      if (live && sub == 0) {
+#pragma unroll
+        for (int k = 0; k < NDIM; ++k) {
+          const uint32_t h = seen_bit(c[k]);
+          atomicOr(&sh.seen[k][h >> 5], 1u << (h & 31u));
+        }
+      }
+    }
+    uint64_t AX = 0, AY = 0, AZ = 0;  // force sums, one per child of a pair
+    const uint64_t MX = pk2(me.x, me.x), MY = pk2(me.y, me.y), MZ = pk2(me.z, me.z);
+    __syncwarp();
+    uint32_t guard = 0;
+    const uint32_t guard_max = 4u * (uint32_t)n + 64u;
+    while (sp > 0) {
+      // gather the first 32 children from the top of the stack, in parallel: lane i reads the i-th
+      // entry from the top, a prefix sum of the entries' child counts places each entry's
+      // children, and a lane's child belongs to the last entry that starts at or before it
+      const bool has = lane < sp;
+      uint4 e = has ? sget(sp - 1 - lane) : make_uint4(0u, 0u, 0u, 0u);
+      if (has && (e.x >= slot_cap || e.y - 1u >= slot_cap - e.x)) {  // a malformed tree: never read past it
+        atomicOr(err, FL_ERR_TREE);
+        e.x = 0u, e.y = 1u;
+      }
+      const uint32_t inc = inclusive_sum(e.y), exc = inc - e.y;
+      const uint32_t avail = __shfl_sync(FL_FULL, inc, 31), total = min(avail, 32u);
+      // entries taken whole leave the stack; one taken in part keeps the rest (the new top)
+      const uint32_t taken = __ballot_sync(FL_FULL, has && inc <= total);
+      if (avail > 32u && has && exc < 32u && inc > 32u)
+        sset(sp - 1 - lane, make_uint4(e.x + (32u - exc), inc - 32u, e.z, e.w));
+      sp -= __popc(taken);
+      const uint32_t starts = __reduce_or_sync(FL_FULL, has && exc < total ? 1u << exc : 0u);
+      const int own = __popc(starts & (below_me | (1u << lane))) - 1;
+      const uint32_t slot = __shfl_sync(FL_FULL, e.x - exc, own) + (uint32_t)lane;
+      const uint32_t my_mask = __shfl_sync(FL_FULL, e.w, own);
+      const uint32_t top = __shfl_sync(FL_FULL, e.z, own);
+      // the lane's child: what it can need of the points
+      const bool ok = (uint32_t)lane < total;
+      float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+      uint2 m = make_uint2(0u, kLeafMark);
+      if (ok) q = __ldg(cdata + slot), m = __ldg(cmeta + slot);
+      const bool lf = m.y == kLeafMark;
+      uint32_t mask = ok && q.w != 0.f ? my_mask : 0u;  // d3 skips a zero value and all it holds
+      if (lf) mask &= ~bit_at(m.x - (uint32_t)base);    // itself
       // a point is never approximated (its sum is the same either way); a cell is opened when
       // even its deepest depth fails the theta test
-      const float topen = lf ? -INFINITY : T0c * pow4neg(D);
-      const float ttop = chain ? T0c * pow4neg(my_top) : topen;
-      const float va = chain ? q.w * alc * damp(NDIM, (int)(D - my_top)) : q.w * alc;
-      float* pa = reinterpret_cast<float*>(spair + (gl & ~1));
-      pa[gl & 1] = q.x, pa[2 + (gl & 1)] = q.y, pa[4 + (gl & 1)] = q.z, pa[6 + (gl & 1)] = va;
-      stest[gl] = make_uint4(__float_as_uint(topen), __float_as_uint(fmaxf(ttop, dminc)), mask, m.x);
-      scold[gl] = make_uint2(m.y, my_top | my_g << 8);
-    } else if (gl < ((jmax + 1) & ~1)) {  // pad the group's batch: a child no lane tests
-      float* pa = reinterpret_cast<float*>(spair + (gl & ~1));
-      pa[gl & 1] = 0.f, pa[2 + (gl & 1)] = 0.f, pa[4 + (gl & 1)] = 0.f, pa[6 + (gl & 1)] = 0.f;
-      stest[gl] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    __syncwarp();
-#pragma unroll 4
-    for (int j = 0; j < jmax; j += 2) {  // two children per round: independent work to overlap
-      const float4 pa = spair[j], pb = spair[j + 1];
-      const uint4 r0 = stest[j], r1 = stest[j + 1];
-      uint64_t DX = sub2(pk2(pa.x, pa.y), MX);
-      uint64_t DY = NDIM > 1 ? sub2(pk2(pa.z, pa.w), MY) : 0ull;
-      uint64_t DZ = NDIM > 2 ? sub2(pk2(pb.x, pb.y), MZ) : 0ull;
-      uint64_t L = mul2(DX, DX);
-      if (NDIM > 1) L = fma2(DY, DY, L);
-      if (NDIM > 2) L = fma2(DZ, DZ, L);
-      const float2 zp = up2(NDIM == 3 ? mul2(mul2(DX, DY), DZ) : NDIM == 2 ? mul2(DX, DY) : DX);
-      float2 l = up2(L);
-      const bool m0 = r0.z & lanebit, m1 = r1.z & lanebit;
-      const bool o0 = m0 && __uint_as_float(r0.x) >= l.x, o1 = m1 && __uint_as_float(r1.x) >= l.y;
-      const bool a0 = m0 && !o0 && (!DMAX || l.x < mydmax2), a1 = m1 && !o1 && (!DMAX || l.y < mydmax2);
-      float v0 = pb.z, v1 = pb.w;
-      const bool c0 = a0 && (l.x <= __uint_as_float(r0.y) || zp.x == 0.f);
-      const bool c1 = a1 && (l.y <= __uint_as_float(r1.y) || zp.y == 0.f);
-      // one warp-uniform branch for everything but the common case (no lane opens either child,
-      // no uncommon case): the common path runs one vote, and never the code inside, even
-      // predicated
-      uint32_t om0 = 0, om1 = 0;
-      if (__any_sync(FL_FULL, c0 || c1 || o0 || o1)) {
-        if (__any_sync(FL_FULL, c0 || c1)) {
-          if (STATS && lane == 0) ++st_rare;
-          float2 dx = up2(DX), dy = up2(DY), dz = up2(DZ);
-          if (c0) {
-            const uint2 k0 = scold[j];
-            rare_case<NDIM>(k0.x, k0.y & 0xffu, r0.w, myT0, mydmin2, myid, myfirst, myng, mycb,
-                            perm, n, mystep, seed, v0, dx.x, dy.x, dz.x, l.x);
-          }
-          if (c1) {
-            const uint2 k1 = scold[j + 1];
-            rare_case<NDIM>(k1.x, k1.y & 0xffu, r1.w, myT0, mydmin2, myid, myfirst, myng, mycb,
-                            perm, n, mystep, seed, v1, dx.y, dy.y, dz.y, l.y);
-          }
-          DX = pk2(dx.x, dx.y), DY = pk2(dy.x, dy.y), DZ = pk2(dz.x, dz.y);
-        }
-        om0 = __ballot_sync(FL_FULL, o0) & gmask;
-        om1 = __ballot_sync(FL_FULL, o1) & gmask;
-        // push the children some lanes of this group must open
-        if (om0) {
-          const uint2 k0 = scold[j];
-          if (sp < kAll && gl == 0)
-            sset(sp, make_uint4(r0.w, k0.x & kCountMask, (((k0.x >> 26) & 31u) + 1u) | (k0.y & ~0xffu), om0));
-          ++sp;
-        }
-        if (om1) {
-          const uint2 k1 = scold[j + 1];
-          if (sp < kAll && gl == 0)
-            sset(sp, make_uint4(r1.w, k1.x & kCountMask, (((k1.x >> 26) & 31u) + 1u) | (k1.y & ~0xffu), om1));
-          ++sp;
-        }
-        if (sp > kAll) {  // beyond the bound on the stack's depth: a malformed tree
-          if (gl == 0) atomicOr(err, FL_ERR_STACK);
-          sp = kAll;
-        }
-        if (STATS && sp > maxsp) maxsp = sp;
+      const uint32_t D = (m.y >> 26) & 31u;
+      const bool chain = !lf && top < D;
+      const float topen = lf ? -INFINITY : T0 * pow4neg(D);
+      const float bound = fmaxf(chain ? T0 * pow4neg(top) : topen, dmin_le);
+      float va = q.w * alpha;
+      if (chain) va *= damp(NDIM, (int)(D - top));
+      const float4 blo = sh.lo, bhi = sh.hi;
+      const float nx = fmaxf(fmaxf(blo.x - q.x, q.x - bhi.x), 0.f);
+      const float ny = NDIM > 1 ? fmaxf(fmaxf(blo.y - q.y, q.y - bhi.y), 0.f) : 0.f;
+      const float nz = NDIM > 2 ? fmaxf(fmaxf(blo.z - q.z, q.z - bhi.z), 0.f) : 0.f;
+      float near2 = nx * nx;
+      if (NDIM > 1) near2 = fmaf(ny, ny, near2);
+      if (NDIM > 2) near2 = fmaf(nz, nz, near2);
+      bool zero = (nx == 0.f) & maybe_seen(sh.seen[0], q.x);
+      if (NDIM > 1) zero |= (ny == 0.f) & maybe_seen(sh.seen[1], q.y);
+      if (NDIM > 2) zero |= (nz == 0.f) & maybe_seen(sh.seen[2], q.z);
+      const bool far = mask == 0u || (!zero && near2 > bound);
+      const bool plain = far || (!zero && near2 > dmin_le && !chain);
+      const uint32_t bfar = __ballot_sync(FL_FULL, far), bplain = __ballot_sync(FL_FULL, plain);
+      {
+        float* pa = reinterpret_cast<float*>(&sh.a[lane >> 1]) + (lane & 1);
+        float* pb = reinterpret_cast<float*>(&sh.b[lane >> 1]) + (lane & 1);
+        float* pt = reinterpret_cast<float*>(&sh.t[lane >> 1]) + (lane & 1);
+        pa[0] = q.x, pa[2] = q.y, pb[0] = q.z, pb[2] = va, pt[0] = topen, pt[2] = bound;
+        sh.mask[lane] = mask;
+        sh.opens[lane] = 0u;
       }
-      const float2 w = up2(mul2(pk2(v0, v1), pk2(rcp_approx(l.x), rcp_approx(l.y))));
-      const uint64_t W = pk2(a0 ? w.x : 0.f, a1 ? w.y : 0.f);
-      AX = fma2(DX, W, AX);
-      if (NDIM > 1) AY = fma2(DY, W, AY);
-      if (NDIM > 2) AZ = fma2(DZ, W, AZ);
+      __syncwarp();
+      // two children per step and lane (per point: S pairs): independent work to overlap. Two steps
+      // of far children are taken at once
+#define FL_WALK_PAIR(jj)                                             \
+  const float4 pa = sh.a[jj], pb = sh.b[jj];                         \
+  const uint2 pm = reinterpret_cast<const uint2*>(sh.mask)[jj];      \
+  uint64_t DX = sub2(pk2(pa.x, pa.y), MX);                           \
+  uint64_t DY = NDIM > 1 ? sub2(pk2(pa.z, pa.w), MY) : 0ull;         \
+  uint64_t DZ = NDIM > 2 ? sub2(pk2(pb.x, pb.y), MZ) : 0ull;         \
+  uint64_t L = mul2(DX, DX);                                         \
+  if (NDIM > 1) L = fma2(DY, DY, L);                                 \
+  if (NDIM > 2) L = fma2(DZ, DZ, L);                                 \
+  float2 l = up2(L);                                                 \
+  const bool m0 = pm.x & lanebit, m1 = pm.y & lanebit;               \
+  bool a0 = m0 && (!DMAX || l.x < dmax2), a1 = m1 && (!DMAX || l.y < dmax2)
+#define FL_WALK_APPLY(v0, v1)                                                                    \
+  do {                                                                                           \
+    const float2 w = up2(mul2(pk2(v0, v1), pk2(rcp_approx(l.x), rcp_approx(l.y))));              \
+    const uint64_t W = pk2(a0 ? w.x : 0.f, a1 ? w.y : 0.f);                                      \
+    AX = fma2(DX, W, AX);                                                                        \
+    if (NDIM > 1) AY = fma2(DY, W, AY);                                                          \
+    if (NDIM > 2) AZ = fma2(DZ, W, AZ);                                                          \
+    if (STATS) st_apply += a0 + a1;                                                              \
+  } while (0)
+      constexpr uint32_t kStep = S == 1 ? 3u : 15u, kTwo = S == 1 ? 15u : 255u;
+      int j = 0;
+      while (j < (int)total) {
+        const int jj = (j >> 1) + sub;
+        if (((bfar >> j) & kTwo) == kTwo) {
+          { FL_WALK_PAIR(jj); FL_WALK_APPLY(pb.z, pb.w); }
+          { FL_WALK_PAIR(jj + S); FL_WALK_APPLY(pb.z, pb.w); }
+          j += 4 * S;
+          continue;
+        }
+        if (((bplain >> j) & kStep) == kStep) {
+          FL_WALK_PAIR(jj);
+          const float4 pt = sh.t[jj];
+          const bool o0 = m0 && pt.x >= l.x, o1 = m1 && pt.y >= l.y;
+          a0 = a0 && !o0, a1 = a1 && !o1;
+          const uint32_t b0 = __ballot_sync(FL_FULL, o0), b1 = __ballot_sync(FL_FULL, o1);
+          reinterpret_cast<uint2*>(sh.opens)[jj] =
+              make_uint2(b0 >> (sub * P & 31) & kPoints, b1 >> (sub * P & 31) & kPoints);
+          FL_WALK_APPLY(pb.z, pb.w);
+          j += 2 * S;
+          continue;
+        }
+        FL_WALK_PAIR(jj);
+        const float4 pt = sh.t[jj];
+        float v0 = pb.z, v1 = pb.w;
+        // the bound covers the theta test too: it is no less than the threshold
+        const float2 zp = up2(NDIM == 3 ? mul2(mul2(DX, DY), DZ) : NDIM == 2 ? mul2(DX, DY) : DX);
+        const bool c0 = l.x <= pt.z || zp.x == 0.f, c1 = l.y <= pt.w || zp.y == 0.f;
+        if (__any_sync(FL_FULL, (m0 && c0) || (m1 && c1))) {
+          const bool o0 = m0 && pt.x >= l.x, o1 = m1 && pt.y >= l.y;
+          a0 = a0 && !o0, a1 = a1 && !o1;
+          const uint32_t b0 = __ballot_sync(FL_FULL, o0), b1 = __ballot_sync(FL_FULL, o1);
+          reinterpret_cast<uint2*>(sh.opens)[jj] =
+              make_uint2(b0 >> (sub * P & 31) & kPoints, b1 >> (sub * P & 31) & kPoints);
+          if (__any_sync(FL_FULL, (a0 && c0) || (a1 && c1))) {
+            if (STATS && lane == 0) ++st_rare;
+            const uint32_t y0 = __shfl_sync(FL_FULL, m.y, 2 * jj), y1 = __shfl_sync(FL_FULL, m.y, 2 * jj + 1);
+            const uint32_t x0 = __shfl_sync(FL_FULL, m.x, 2 * jj), x1 = __shfl_sync(FL_FULL, m.x, 2 * jj + 1);
+            const uint32_t p0 = __shfl_sync(FL_FULL, top, 2 * jj), p1 = __shfl_sync(FL_FULL, top, 2 * jj + 1);
+            float2 dx = up2(DX), dy = up2(DY), dz = up2(DZ);
+            if (a0 && c0)
+              rare_case<NDIM>(y0, p0, x0, T0, dmin2, myid, gfirst, gcount, gcells, perm, n, gstep,
+                              seed, v0, dx.x, dy.x, dz.x, l.x);
+            if (a1 && c1)
+              rare_case<NDIM>(y1, p1, x1, T0, dmin2, myid, gfirst, gcount, gcells, perm, n, gstep,
+                              seed, v1, dx.y, dy.y, dz.y, l.y);
+            DX = pk2(dx.x, dx.y), DY = pk2(dy.x, dy.y), DZ = pk2(dz.x, dz.y);
+          }
+        }
+        FL_WALK_APPLY(v0, v1);
+        j += 2 * S;
+      }
+#undef FL_WALK_PAIR
+#undef FL_WALK_APPLY
+      __syncwarp();
+      // the children some points must open go on the stack, in child order
+      const uint32_t opens = sh.opens[lane];
+      const uint32_t pushes = __ballot_sync(FL_FULL, opens != 0u);
+      if (opens) {
+        const int to = sp + __popc(pushes & below_me);
+        if (to < kAll) sset(to, make_uint4(m.x, m.y & kCountMask, D + 1u, opens));
+      }
+      sp += __popc(pushes);
+      if (sp > kAll) {  // beyond the bound on the stack's depth: a malformed tree
+        if (lane == 0) atomicOr(err, FL_ERR_STACK);
+        sp = kAll;
+      }
       if (STATS) {
-        const uint32_t ap = __ballot_sync(FL_FULL, a0) & gmask, aq = __ballot_sync(FL_FULL, a1) & gmask;
-        if (gl == 0) {
-          if (j < total) st_tests += G, st_useful += __popc(r0.z & gmask);
-          if (j + 1 < total) st_tests += G, st_useful += __popc(r1.z & gmask);
-          st_open += __popc(om0) + __popc(om1);
-          st_apply += __popc(ap) + __popc(aq);
-        }
+        if (ok) st_tests += P, st_useful += __popc(mask), st_open += __popc(opens);
+        if (sp > maxsp) maxsp = sp;
+      }
+      __syncwarp();
+      if (++guard > guard_max) {
+        if (lane == 0) atomicOr(err, FL_ERR_STACK);
+        break;
       }
     }
-    __syncwarp();
-    if (++guard > guard_max) {
-      if (lane == 0) atomicOr(err, FL_ERR_STACK);
-      break;
-    }
-  }
-  if (live) {
     const float2 ax2 = up2(AX), ay2 = up2(AY), az2 = up2(AZ);
-    float4 v = vel[myid];
-    v.x += ax2.x + ax2.y;
-    if (NDIM > 1) v.y += ay2.x + ay2.y;
-    if (NDIM > 2) v.z += az2.x + az2.y;
-    vel[myid] = v;
-  }
-  __syncwarp();
-  wi = lane == 0 ? (int)atomicAdd(work, 1u) : 0;
-  wi = __shfl_sync(FL_FULL, wi, 0);
+    float ax = ax2.x + ax2.y, ay = ay2.x + ay2.y, az = az2.x + az2.y;
+#pragma unroll
+    for (int o = P; o < 32; o <<= 1) {  // a point's lanes
+      ax += __shfl_xor_sync(FL_FULL, ax, o);
+      if (NDIM > 1) ay += __shfl_xor_sync(FL_FULL, ay, o);
+      if (NDIM > 2) az += __shfl_xor_sync(FL_FULL, az, o);
+    }
+    if (live && sub == 0) {
+      float4 v = vel[myid];
+      v.x += ax;
+      if (NDIM > 1) v.y += ay;
+      if (NDIM > 2) v.z += az;
+      vel[myid] = v;
+    }
+    __syncwarp();
+    wi = lane == 0 ? (int)atomicAdd(work, 1u) : 0;
+    wi = __shfl_sync(FL_FULL, wi, 0);
   }
   // every warp ends on one claim past the last group; the last of those claims puts the counter
   // back to 0 for the next launch (no other warp touches it after its own last claim)
-  if (lane == 0 && wi == nwarps + (int)(gridDim.x * kWalkWarps) - 1) *work = 0u;
+  if (lane == 0 && wi == ngroups + (int)(gridDim.x * kWalkWarps) - 1) *work = 0u;
   if (STATS) {
-    if (gl == 0) {
-      atomicAdd(stats, st_tests);
-      atomicAdd(stats + 1, st_useful);
-      atomicMax(stats + 2, (unsigned long long)maxsp);
-      atomicAdd(stats + 3, st_open);
-      atomicAdd(stats + 4, st_apply);
-    }
+    atomicAdd(stats, st_tests);
+    atomicAdd(stats + 1, st_useful);
+    atomicMax(stats + 2, (unsigned long long)maxsp);
+    atomicAdd(stats + 3, st_open);
+    atomicAdd(stats + 4, st_apply);
     if (lane == 0) atomicAdd(stats + 5, st_rare);
   }
 }
@@ -1757,7 +1822,8 @@ void fl_launch_walk(const FlTreeBufs* t, const uint32_t* perm, const float* cube
                     uint32_t seed, uint32_t* err, unsigned long long* stats, int group,
                     cudaStream_t st, FlSegs segs, const FlTick* tk) {
   const int n = t->n;
-  const int warps = segs.graphs ? segs.ngroups : (n + 31) / 32;
+  const int points = group == 16 && !segs.graphs ? 16 : 32;
+  const int groups = segs.graphs ? segs.ngroups : (n + points - 1) / points;
   // a persistent grid of the blocks that fit on the device at once (and that the spill buffer
   // has regions for), each warp walking every (grid)-th group of 32 points
   const int cap = t->walk_slots / kWalkWarps;
@@ -1774,7 +1840,7 @@ void fl_launch_walk(const FlTreeBufs* t, const uint32_t* perm, const float* cube
     if (g < 1) g = 1;                                                                          \
     k_walk<D, G, S, M, B><<<g, kWalkThreads, 0, st>>>(                                         \
         t->child_data, t->child_meta, t->leaf, perm, cube, vel, n, alpha, theta2,              \
-        (float)dmin2, fmax2, step, seed, err, stats, t->spill, warps, t->work, segs, tk);      \
+        (float)dmin2, fmax2, step, seed, err, stats, t->spill, groups, t->work, segs, tk);      \
   } while (0)
 #define FL_WALK(D, G)                                                                          \
   do {                                                                                         \
