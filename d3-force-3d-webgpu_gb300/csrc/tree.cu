@@ -36,6 +36,7 @@
 //              cells that some point must open are pushed with the mask of those points.
 //
 // Points with the same code at the finest level share the deepest cell as its children.
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <atomic>
@@ -1544,64 +1545,182 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
   }
 }
 
-// Exact all-pairs sum (theta ~ 0; src/gpu/passes/manyBody.js:5-16 semantics): each block
-// streams the points through shared memory in tiles.
-constexpr int kPairThreads = 256;
-__global__ void __launch_bounds__(kPairThreads) k_allpairs(const float4* __restrict__ pos,
-                                                           const float* __restrict__ strength,
-                                                           float4* __restrict__ vel, int n,
-                                                           int ndim, float alpha, float dmin2,
-                                                           float dmax2, uint32_t step,
-                                                           uint32_t seed, int split,
-                                                           const FlTick* __restrict__ tk) {
+// Exact all-pairs sum (theta ~ 0; src/gpu/passes/manyBody.js:5-16 semantics). A cluster of up to 8
+// blocks sums the forces on 32 Q points: every warp holds the same points, Q per lane, and takes
+// every (warps of the cluster)-th tile of 32 sources, which its lanes load and lay out in shared
+// memory as pairs for the f32x2 arithmetic. Four sources at a time, for every point of the lane,
+// are tested for what is not the common case (the point itself, distanceMin, a zero component)
+// by the least of their squared distances and components, with one vote; such a four is summed
+// again source by source. The warps' sums are added in a fixed order, in shared memory and then
+// over the cluster's.
+//
+// Bound by the FP32 pipe and instruction issue: a pair of sources takes 10 packed instructions of
+// 2 cycles each and 25 issue slots. 20,000 points in 3D: 212 us (110 is the packed instructions
+// alone), where one thread per point and sixteenth of the sources, each source tested in scalars,
+// took 757; 4,000 points 64 -> 20, 1,000 points 21 -> 10. Blocks of 128 threads: 256 wait longer
+// for their slowest warp (249 us).
+constexpr int kPairThreads = 128;
+constexpr int kPairWarps = kPairThreads / 32;
+constexpr int kPairClusterMax = 8;
+constexpr int kPairTwoPoints = 10000;  // more points than this: two per lane
+
+// One source's force on a point, every case.
+template <int NDIM, bool DMAX>
+__device__ __forceinline__ void pair_term(float4 me, uint32_t i, float4 o, uint32_t other,
+                                          float dmin2, float dmax2, uint32_t step, uint32_t seed,
+                                          float& ax, float& ay, float& az) {
+  if (other == i || o.w == 0.f) return;
+  float dx = o.x - me.x, dy = NDIM > 1 ? o.y - me.y : 0.f, dz = NDIM > 2 ? o.z - me.z : 0.f;
+  float l = dx * dx;
+  if (NDIM > 1) l = fmaf(dy, dy, l);
+  if (NDIM > 2) l = fmaf(dz, dz, l);
+  if (DMAX && l >= dmax2) return;
+  if (dx == 0.f) dx = fl::jiggle(i, other, 0, step, seed), l += dx * dx;
+  if (NDIM > 1 && dy == 0.f) dy = fl::jiggle(i, other, 1, step, seed), l += dy * dy;
+  if (NDIM > 2 && dz == 0.f) dz = fl::jiggle(i, other, 2, step, seed), l += dz * dz;
+  if (l < dmin2) l = sqrtf(dmin2 * l);
+  const float w = o.w * rcp_approx(l);
+  ax = fmaf(dx, w, ax), ay = fmaf(dy, w, ay), az = fmaf(dz, w, az);
+}
+
+template <int NDIM, int Q, bool DMAX>
+__global__ void __launch_bounds__(kPairThreads) k_allpairs(
+    const float4* __restrict__ pos, const float* __restrict__ strength, float4* __restrict__ vel,
+    int n, float alpha, float dmin2, float dmax2, uint32_t step, uint32_t seed,
+    const FlTick* __restrict__ tk) {
   if (tk) alpha = tk->alpha, step = tk->step, seed = tk->seed;
-  __shared__ float4 tile[kPairThreads];
-  __shared__ float3 part[kPairThreads];
-  const int per = kPairThreads / split;
-  const int lane = threadIdx.x % split;
-  const int i = blockIdx.x * per + threadIdx.x / split;
-  const bool live = i < n;
-  float4 me = live ? pos[i] : make_float4(0, 0, 0, 0);
-  float ax = 0.f, ay = 0.f, az = 0.f;
-  for (int base = 0; base < n; base += kPairThreads) {
-    const int j = base + threadIdx.x;
-    float4 q = make_float4(0, 0, 0, 0);
-    if (j < n) q = pos[j], q.w = strength[j];
-    tile[threadIdx.x] = q;
-    __syncthreads();
-    const int cnt = n - base < kPairThreads ? n - base : kPairThreads;
-    if (live) {
-      for (int k = lane; k < cnt; k += split) {
-        const float4 o = tile[k];
-        if (base + k == i || o.w == 0.f) continue;
-        float dx = o.x - me.x, dy = ndim > 1 ? o.y - me.y : 0.f, dz = ndim > 2 ? o.z - me.z : 0.f;
-        float l = dx * dx + dy * dy + dz * dz;
-        if (l >= dmax2) continue;
-        if (dx == 0.f || (ndim > 1 && dy == 0.f) || (ndim > 2 && dz == 0.f)) {
-          const uint32_t other = (uint32_t)(base + k);
-          if (dx == 0.f) dx = fl::jiggle(i, other, 0, step, seed), l += dx * dx;
-          if (ndim > 1 && dy == 0.f) dy = fl::jiggle(i, other, 1, step, seed), l += dy * dy;
-          if (ndim > 2 && dz == 0.f) dz = fl::jiggle(i, other, 2, step, seed), l += dz * dz;
-        }
-        if (l < dmin2) l = sqrtf(dmin2 * l);
-        const float w = __fdividef(o.w * alpha, l);
-        ax += dx * w, ay += dy * w, az += dz * w;
-      }
+  __shared__ float4 s_a[kPairWarps][16], s_b[kPairWarps][16];  // {x, x', y, y'}, {z, z', s, s'}
+  __shared__ float s_part[kPairWarps][3][32 * Q];
+  __shared__ float s_sum[3][32 * Q];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first = (int)(blockIdx.x / blocks) * 32 * Q;
+  float4 me[Q];
+  uint64_t MX[Q], MY[Q], MZ[Q], AX[Q], AY[Q], AZ[Q];
+#pragma unroll
+  for (int p = 0; p < Q; ++p) {
+    const int i = first + 32 * p + lane;
+    me[p] = i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    MX[p] = pk2(me[p].x, me[p].x), MY[p] = pk2(me[p].y, me[p].y), MZ[p] = pk2(me[p].z, me[p].z);
+    AX[p] = AY[p] = AZ[p] = 0;
+  }
+  constexpr int K = 2;  // pairs of sources at a time
+  const float close = fmaxf(below(dmin2), 0.f);  // l <= close: distanceMin, or no distance at all
+  float4* sa = s_a[warp];
+  float4* sb = s_b[warp];
+  for (int base = 32 * (rank * kPairWarps + warp); base < n; base += 32 * kPairWarps * blocks) {
+    const int j = base + lane;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j < n) o = pos[j], o.w = strength[j] * alpha;
+    __syncwarp();
+    {
+      float* pa = reinterpret_cast<float*>(&sa[lane >> 1]) + (lane & 1);
+      float* pb = reinterpret_cast<float*>(&sb[lane >> 1]) + (lane & 1);
+      pa[0] = o.x, pa[2] = o.y, pb[0] = o.z, pb[2] = o.w;
     }
-    __syncthreads();
+    __syncwarp();
+#pragma unroll 1
+    for (int k = 0; k < 16; k += K) {
+      float4 a[K], b[K];
+      uint64_t DX[Q][K], DY[Q][K], DZ[Q][K];
+      float2 l[Q][K];
+      float lmin = INFINITY, cmin = INFINITY;
+#pragma unroll
+      for (int c = 0; c < K; ++c) a[c] = sa[k + c], b[c] = sb[k + c];
+#pragma unroll
+      for (int p = 0; p < Q; ++p)
+#pragma unroll
+        for (int c = 0; c < K; ++c) {
+          DX[p][c] = sub2(pk2(a[c].x, a[c].y), MX[p]);
+          DY[p][c] = NDIM > 1 ? sub2(pk2(a[c].z, a[c].w), MY[p]) : 0ull;
+          DZ[p][c] = NDIM > 2 ? sub2(pk2(b[c].x, b[c].y), MZ[p]) : 0ull;
+          uint64_t L = mul2(DX[p][c], DX[p][c]);
+          if (NDIM > 1) L = fma2(DY[p][c], DY[p][c], L);
+          if (NDIM > 2) L = fma2(DZ[p][c], DZ[p][c], L);
+          l[p][c] = up2(L);
+          const float2 dx = up2(DX[p][c]), dy = up2(DY[p][c]), dz = up2(DZ[p][c]);
+          lmin = fminf(fminf(lmin, l[p][c].x), l[p][c].y);
+          cmin = fminf(fminf(cmin, fabsf(dx.x)), fabsf(dx.y));
+          if (NDIM > 1) cmin = fminf(fminf(cmin, fabsf(dy.x)), fabsf(dy.y));
+          if (NDIM > 2) cmin = fminf(fminf(cmin, fabsf(dz.x)), fabsf(dz.y));
+        }
+      bool odd = lmin <= close || cmin == 0.f;
+      // in a small layout mostly the point itself: then as if infinitely far (in a large one it is
+      // met too seldom for what the test costs in registers)
+      if (Q == 1 && __any_sync(FL_FULL, odd)) {
+        odd = false;
+#pragma unroll
+        for (int c = 0; c < K; ++c) {
+          const int self = first + lane - (base + 2 * (k + c));
+          const float2 dx = up2(DX[0][c]), dy = up2(DY[0][c]), dz = up2(DZ[0][c]);
+          if (self == 0) l[0][c].x = INFINITY;
+          else odd |= l[0][c].x <= close || dx.x == 0.f || (NDIM > 1 && dy.x == 0.f) || (NDIM > 2 && dz.x == 0.f);
+          if (self == 1) l[0][c].y = INFINITY;
+          else odd |= l[0][c].y <= close || dx.y == 0.f || (NDIM > 1 && dy.y == 0.f) || (NDIM > 2 && dz.y == 0.f);
+        }
+      }
+      if (__any_sync(FL_FULL, odd)) {
+#pragma unroll
+        for (int p = 0; p < Q; ++p) {
+          float2 ax = up2(AX[p]), ay = up2(AY[p]), az = up2(AZ[p]);
+          const uint32_t i = (uint32_t)(first + 32 * p + lane);
+#pragma unroll 1
+          for (int c = 0; c < K; ++c) {
+            const float4 u = sa[k + c], v = sb[k + c];
+            const uint32_t at = (uint32_t)(base + 2 * (k + c));
+            pair_term<NDIM, DMAX>(me[p], i, make_float4(u.x, u.z, v.x, v.z), at, dmin2, dmax2, step, seed, ax.x, ay.x, az.x);
+            pair_term<NDIM, DMAX>(me[p], i, make_float4(u.y, u.w, v.y, v.w), at + 1, dmin2, dmax2, step, seed, ax.y, ay.y, az.y);
+          }
+          AX[p] = pk2(ax.x, ax.y), AY[p] = pk2(ay.x, ay.y), AZ[p] = pk2(az.x, az.y);
+        }
+        continue;
+      }
+#pragma unroll
+      for (int p = 0; p < Q; ++p)
+#pragma unroll
+        for (int c = 0; c < K; ++c) {
+          uint64_t W = mul2(pk2(b[c].z, b[c].w), pk2(rcp_approx(l[p][c].x), rcp_approx(l[p][c].y)));
+          if (DMAX) {
+            const float2 w = up2(W);
+            W = pk2(l[p][c].x < dmax2 ? w.x : 0.f, l[p][c].y < dmax2 ? w.y : 0.f);
+          }
+          AX[p] = fma2(DX[p][c], W, AX[p]);
+          if (NDIM > 1) AY[p] = fma2(DY[p][c], W, AY[p]);
+          if (NDIM > 2) AZ[p] = fma2(DZ[p][c], W, AZ[p]);
+        }
+    }
   }
-  part[threadIdx.x] = make_float3(ax, ay, az);
+#pragma unroll
+  for (int p = 0; p < Q; ++p) {
+    const float2 ax = up2(AX[p]), ay = up2(AY[p]), az = up2(AZ[p]);
+    s_part[warp][0][32 * p + lane] = ax.x + ax.y;
+    s_part[warp][1][32 * p + lane] = ay.x + ay.y;
+    s_part[warp][2][32 * p + lane] = az.x + az.y;
+  }
   __syncthreads();
-  if (!live || lane != 0) return;
-  for (int s = 1; s < split; ++s) {
-    float3 p = part[threadIdx.x + s];
-    ax += p.x, ay += p.y, az += p.z;
+  for (int t = threadIdx.x; t < 3 * 32 * Q; t += kPairThreads) {
+    const int c = t / (32 * Q), x = t % (32 * Q);
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPairWarps; ++w) sum += s_part[w][c][x];
+    s_sum[c][x] = sum;
   }
-  float4 v = vel[i];
-  v.x += ax;
-  if (ndim > 1) v.y += ay;
-  if (ndim > 2) v.z += az;
-  vel[i] = v;
+  if (blocks > 1) cluster.sync();
+  else __syncthreads();
+  const int i = first + (int)threadIdx.x;
+  if (rank == 0 && threadIdx.x < 32 * Q && i < n) {
+    float4 v = vel[i];
+    float a[3] = {0.f, 0.f, 0.f};
+    for (int r = 0; r < blocks; ++r)
+#pragma unroll
+      for (int c = 0; c < NDIM; ++c) a[c] += cluster.map_shared_rank(&s_sum[c][threadIdx.x], r)[0];
+    v.x += a[0];
+    if (NDIM > 1) v.y += a[1];
+    if (NDIM > 2) v.z += a[2];
+    vel[i] = v;
+  }
+  if (blocks > 1) cluster.sync();  // no block leaves while its sums are read
 }
 
 }  // namespace
@@ -1901,13 +2020,39 @@ void fl_launch_walk(const FlTreeBufs* t, const uint32_t* perm, const float* cube
 void fl_launch_allpairs(const float4* pos, const float* strength, float4* vel, int n, int ndim,
                         float alpha, float dmin2, float dmax2, uint32_t step, uint32_t seed,
                         cudaStream_t st, const FlTick* tk) {
-  // threads per point: enough threads in flight for small graphs (2^18 in all), at most 16
-  int split = 1;
-  while (split < 16 && (int64_t)n * split < (1 << 18)) split *= 2;
-  const int per = kPairThreads / split;
-  const int g = (n + per - 1) / per;
-  k_allpairs<<<g < 1 ? 1 : g, kPairThreads, 0, st>>>(pos, strength, vel, n, ndim, alpha, dmin2,
-                                                     dmax2, step, seed, split, tk);
+  // two points per lane halve the reads of shared memory, one spreads a small layout over more
+  // warps: 8,000 points take 49 us with one and 55 with two, 20,000 268 and 212. Clusters of 8
+  // blocks, unless fewer give every SM 16 blocks (4 at 20,000 points: 215 us) or a warp has no tile
+  const int q = n > kPairTwoPoints ? 2 : 1;
+  const int units = (n + 32 * q - 1) / (32 * q);
+  int blocks = kPairClusterMax;
+  while (blocks > 1 && ((int64_t)units * blocks / 2 >= (int64_t)16 * fl_sms() || n <= 32 * kPairWarps * (blocks / 2)))
+    blocks /= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(units < 1 ? 1 : units) * (unsigned)blocks);
+  cfg.blockDim = dim3(kPairThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)blocks, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr, cfg.numAttrs = blocks > 1 ? 1 : 0;
+#define FL_PAIRS(D, Q, M) \
+  cudaLaunchKernelEx(&cfg, k_allpairs<D, Q, M>, pos, strength, vel, n, alpha, dmin2, dmax2, step, seed, tk)
+#define FL_PAIRS_DIM(D)                                              \
+  do {                                                               \
+    if (dmax2 < INFINITY) {                                          \
+      if (q == 2) FL_PAIRS(D, 2, true);                              \
+      else FL_PAIRS(D, 1, true);                                     \
+    } else {                                                         \
+      if (q == 2) FL_PAIRS(D, 2, false);                             \
+      else FL_PAIRS(D, 1, false);                                    \
+    }                                                                \
+  } while (0)
+  if (ndim == 3) FL_PAIRS_DIM(3);
+  else if (ndim == 2) FL_PAIRS_DIM(2);
+  else FL_PAIRS_DIM(1);
+#undef FL_PAIRS_DIM
+#undef FL_PAIRS
 }
 
 void fl_launch_bgraph(int graphs, int ndim, const int32_t* off, const FlReduce* red,
