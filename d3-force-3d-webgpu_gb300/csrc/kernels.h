@@ -83,19 +83,20 @@ struct FlSortBufs {
   uint32_t* longs;     // [longs_cap] first positions of the runs the fix-up sorts in one block
   uint32_t longs_cap;
   int64_t cap;         // pairs the buffers hold
-  int64_t tiles_cap;   // tiles of kSortTileSmall pairs the look-back words have room for
+  int64_t tiles_cap;   // tiles the look-back words have room for
   // 0, or a test of the bounded look-back: every wait gives up after this many polls, and the
   // first digit pass withholds tile 0's counts, so that the waits run out (the tiles that gave
   // up count their predecessors' keys themselves: the result stays exact, FL_ERR_LOOKBACK is set)
   uint32_t test_spins;
 };
 constexpr int kSortCounters = 16;
-// A onesweep tile: 256 threads x kSortItems pairs for up to kSortSmallMax pairs (small sorts
-// take more, shorter tiles: the time of a pass is that of one tile's steps); above, 1024 threads
-// x 5 to kSortItems pairs, as few as give every SM a tile (fl_sort_tile).
-constexpr int kSortThreads = 1024, kSortThreadsSmall = 256, kSortItems = 8;
-constexpr int kSortTileSmall = kSortThreadsSmall * kSortItems;
-constexpr int64_t kSortSmallMax = 131072;
+// A onesweep tile: 256 threads x 2 to 4 pairs for up to kSortSmallMax pairs, at most kSortTilesSmall
+// tiles; above, 512 or 1024 threads x 5 to kSortItems pairs (sort_shape).
+struct FlSortShape {
+  int threads, items;
+};
+constexpr int kSortItems = 8, kSortItemsMin = 2, kSortTilesSmall = 128, kSortTileMid = 512 * 5;
+constexpr int64_t kSortSmallMax = 256 * 4 * kSortTilesSmall;  // 131,072
 int fl_sort_tile(int64_t n);  // pairs per tile for a sort of n pairs
 int fl_sms();        // SMs of the current device (cached per device)
 size_t fl_sort_bytes(int64_t n);

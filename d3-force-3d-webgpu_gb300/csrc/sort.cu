@@ -381,7 +381,11 @@ int64_t tiles_for(int64_t n) {
   const int64_t t = fl_sort_tile(n);
   return (n + t - 1) / t;
 }
-int64_t tiles_cap_for(int64_t cap) { return (cap + kSortTileSmall - 1) / kSortTileSmall; }
+// the most tiles a sort of up to cap pairs has
+int64_t tiles_cap_for(int64_t cap) {
+  const int64_t t = (cap + kSortTileMid - 1) / kSortTileMid;
+  return t > kSortTilesSmall ? t : kSortTilesSmall;
+}
 
 // True the first time it is called on the current device for `done` (a kernel's shared-memory
 // limit is raised once per device, and on the first launch, which is never inside a capture).
@@ -448,17 +452,28 @@ __global__ void __launch_bounds__(kRankWarps * 32) k_ranksort(const uint64_t* __
 
 }  // namespace
 
-// Keys per thread of a pass's tiles of 1024 threads: as few as fill every SM with one tile (the
-// pass then takes one wave, each tile's time growing with its keys), from 5 up to 8 (beyond
-// 152 SMs x 8 x 1024 = 1.2 M keys, more than one wave of the largest tiles).
-static int sort_items(int64_t n) {
-  const int64_t per_sm = (int64_t)fl_sms() * kSortThreads;
-  int64_t it = (n + per_sm - 1) / per_sm;
-  return it < 5 ? 5 : it > kSortItems ? kSortItems : (int)it;
+// The tile of a sort of n pairs: as few keys as give one wave of tiles, in blocks as small as hold
+// them. A pass takes the time of one tile's steps, which grows with its keys and with its warps, plus
+// the look-back, which grows with the tiles. A pass of the tree's sort (ncu) went, against tiles of
+// 2,048 keys up to 131,072 and 1024 x 5 to 8 above, from 7.6 us to 5.8 at 20k keys, 8.5 to 7.1 at 50k,
+// 11.6 to 9.4 at 300k. From 131,072 to 262,144 keys 256 x 5 to 8 is as fast alone, but 1.5 % slower for
+// a tick at 200k beside others'. Above one wave of the largest tiles two blocks of 512 fit an SM, and
+// one's phases fill the other's: 24.2 us against 27.5 at 1.6M, 38 against 40 at 3M.
+static FlSortShape sort_shape(int64_t n) {
+  if (n <= kSortSmallMax) {
+    const int64_t it = (n + kSortTilesSmall * 256 - 1) / (kSortTilesSmall * 256);
+    return {256, it < kSortItemsMin ? kSortItemsMin : (int)it};
+  }
+  const int64_t sms = fl_sms();
+  if (n > sms * 1024 * kSortItems) return {512, 6};
+  const int threads = n <= sms * 512 * kSortItems ? 512 : 1024;
+  const int64_t it = (n + sms * threads - 1) / (sms * threads);
+  return {threads, it < 5 ? 5 : (int)it};
 }
 
 int fl_sort_tile(int64_t n) {
-  return n <= kSortSmallMax ? kSortTileSmall : kSortThreads * sort_items(n);
+  const FlSortShape s = sort_shape(n);
+  return s.threads * s.items;
 }
 
 // The SM count of the current device, queried once per device index. The cache entries are
@@ -527,6 +542,7 @@ int fl_sort_passes(const FlSortBufs* b, int64_t n, int lo_bit, uint32_t* err, cu
   int cur = 0;
   if (n <= 0) return 0;
   const int64_t tiles = tiles_for(n);
+  const FlSortShape shape = sort_shape(n);
   // the test of the bounded wait (b->test_spins > 0): the first pass withholds tile 0's counts
   const uint32_t limit = b->test_spins ? b->test_spins : FL_SPIN_LIMIT;
   for (int p = 0; p < passes; ++p) {
@@ -535,12 +551,18 @@ int fl_sort_passes(const FlSortBufs* b, int64_t n, int lo_bit, uint32_t* err, cu
 #define FL_PASS(T, I)                                                                          \
   launch_pass<T, I>(b->keys[cur], b->vals[cur], b->keys[1 - cur], b->vals[1 - cur], n,            \
                     lo_bit + 8 * p, b->hist + p * 256, status, b->counters + p, err, limit, hold, st)
-    switch (fl_sort_tile(n)) {
-      case kSortTileSmall: FL_PASS(kSortThreadsSmall, kSortItems); break;
-      case 5 * kSortThreads: FL_PASS(kSortThreads, 5); break;
-      case 6 * kSortThreads: FL_PASS(kSortThreads, 6); break;
-      case 7 * kSortThreads: FL_PASS(kSortThreads, 7); break;
-      default: FL_PASS(kSortThreads, 8); break;
+    switch (shape.threads * 16 + shape.items) {
+      case 256 * 16 + 2: FL_PASS(256, 2); break;
+      case 256 * 16 + 3: FL_PASS(256, 3); break;
+      case 256 * 16 + 4: FL_PASS(256, 4); break;
+      case 512 * 16 + 5: FL_PASS(512, 5); break;
+      case 512 * 16 + 6: FL_PASS(512, 6); break;
+      case 512 * 16 + 7: FL_PASS(512, 7); break;
+      case 512 * 16 + 8: FL_PASS(512, 8); break;
+      case 1024 * 16 + 5: FL_PASS(1024, 5); break;
+      case 1024 * 16 + 6: FL_PASS(1024, 6); break;
+      case 1024 * 16 + 7: FL_PASS(1024, 7); break;
+      default: FL_PASS(1024, 8); break;
     }
 #undef FL_PASS
     ++*launches;

@@ -27,8 +27,8 @@ void fl_set_sim_free_error(const std::string& msg);  // engine.cu: the message o
 namespace {
 
 constexpr int64_t kMaxPairs = FL_SORT_NOALLOC_MAX_PAIRS;
-constexpr int64_t kTile = kSortTileSmall;  // the smallest onesweep tile: the most tiles
-constexpr int64_t kTiles = (kMaxPairs + kTile - 1) / kTile;
+constexpr int64_t kTiles = kSortTilesSmall;  // the most tiles of a sort of up to kMaxPairs pairs
+static_assert(kMaxPairs <= kTiles * kSortTileMid, "more pairs have more tiles");
 constexpr size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kErrOff = 0;
 constexpr size_t kKeysOff = 256;
