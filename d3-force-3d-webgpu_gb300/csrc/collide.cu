@@ -9,9 +9,11 @@
 // the same or adjacent cells. Each cell maps to a slot of a table of 2^bits >= 2n slots: cells
 // are grouped in blocks (4^3, 8^2 or 64 cells) whose cells take consecutive slots in Morton
 // order from a hashed block offset, so the sort by slot keeps nearby cells nearby. Two cells
-// sharing a slot only cost extra distance tests; a node looks through each distinct slot of its
-// 3^d neighbour cells once. Run starts are never cleared: a start is trusted only if the sorted
-// keys confirm it.
+// sharing a slot only cost extra distance tests; the 3^d neighbour cells of a node never share one
+// (cells of one place in their blocks are at least a block's side apart). A slot's run of sorted
+// nodes, [start, end), is written when it has one and never cleared: its words carry the low bits of
+// the tick's step, and a run whose bits match is trusted only if the sorted keys confirm it. (If
+// the slot has nodes now, its run was written now.)
 #include "kernels.h"
 
 namespace {
@@ -20,24 +22,29 @@ constexpr int kThreads = 256;
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-__device__ __forceinline__ void pair_push(float3 me, float ri2, float ri, float4 o, uint32_t idi,
-                                          uint32_t idj, int ndim, float strength, uint32_t step,
+// One pair's push on node idi (radius ri), if they overlap. Every rounding is spelt out, so that a
+// pair pushes the same bit for bit wherever it is found. (The other node's id, perm[t] - first, or t
+// itself without perm, is read only for a jiggle.)
+__device__ __forceinline__ void pair_push(float3 me, float ri, float4 o, uint32_t idi,
+                                          const uint32_t* __restrict__ perm, uint32_t t,
+                                          uint32_t first, int ndim, float strength, uint32_t step,
                                           uint32_t seed, float3& acc) {
   const float rj = o.w, r = ri + rj;
   float dx = me.x - o.x, dy = ndim > 1 ? me.y - o.y : 0.f, dz = ndim > 2 ? me.z - o.z : 0.f;
-  float l = dx * dx + dy * dy + dz * dz;
+  float l = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
   if (!(l < r * r)) return;
   if (dx == 0.f || (ndim > 1 && dy == 0.f) || (ndim > 2 && dz == 0.f)) {
-    if (dx == 0.f) dx = fl::jiggle(idi, idj, 0, step, seed), l += dx * dx;
-    if (ndim > 1 && dy == 0.f) dy = fl::jiggle(idi, idj, 1, step, seed), l += dy * dy;
-    if (ndim > 2 && dz == 0.f) dz = fl::jiggle(idi, idj, 2, step, seed), l += dz * dz;
+    const uint32_t idj = perm ? perm[t] - first : t;
+    if (dx == 0.f) dx = fl::jiggle(idi, idj, 0, step, seed), l = __fmaf_rn(dx, dx, l);
+    if (ndim > 1 && dy == 0.f) dy = fl::jiggle(idi, idj, 1, step, seed), l = __fmaf_rn(dy, dy, l);
+    if (ndim > 2 && dz == 0.f) dz = fl::jiggle(idi, idj, 2, step, seed), l = __fmaf_rn(dz, dz, l);
   }
   const float len = sqrtf(l);
-  const float k = (r - len) / len * strength;
-  const float rj2 = rj * rj, w = rj2 / (ri2 + rj2);
-  acc.x += dx * k * w;
-  acc.y += dy * k * w;
-  acc.z += dz * k * w;
+  const float k = __fmul_rn(__fdiv_rn(__fsub_rn(r, len), len), strength);
+  const float rj2 = __fmul_rn(rj, rj), w = __fdiv_rn(rj2, __fmaf_rn(ri, ri, rj2));
+  acc.x = __fmaf_rn(__fmul_rn(dx, k), w, acc.x);
+  acc.y = __fmaf_rn(__fmul_rn(dy, k), w, acc.y);
+  acc.z = __fmaf_rn(__fmul_rn(dz, k), w, acc.z);
 }
 
 __global__ void __launch_bounds__(kThreads) k_collide_allpairs(
@@ -55,7 +62,6 @@ __global__ void __launch_bounds__(kThreads) k_collide_allpairs(
   float ri = 0.f;
   if (live) p = pos[i], v = vel_in[i], ri = radius[i];
   const float3 me = make_float3(p.x + v.x, p.y + v.y, p.z + v.z);
-  const float ri2 = ri * ri;
   float3 acc = make_float3(0.f, 0.f, 0.f);
   for (int base = 0; base < n; base += kThreads) {
     const int j = base + threadIdx.x;
@@ -69,7 +75,8 @@ __global__ void __launch_bounds__(kThreads) k_collide_allpairs(
     const int cnt = n - base < kThreads ? n - base : kThreads;
     if (live)
       for (int k = lane; k < cnt; k += split)
-        if (base + k != i) pair_push(me, ri2, ri, tile[k], i, base + k, ndim, strength, step, seed, acc);
+        if (base + k != i)
+          pair_push(me, ri, tile[k], i, nullptr, base + k, 0u, ndim, strength, step, seed, acc);
     __syncthreads();
   }
   part[threadIdx.x] = acc;
@@ -109,11 +116,99 @@ __device__ __forceinline__ uint32_t cell_slot(int cx, int cy, int cz, int ndim, 
   return ((h << 6) + w) & mask;
 }
 
+// A table entry's two words: the run's start and end (26 bits), tagged with the tick.
+constexpr uint32_t kRunMask = (1u << 26) - 1;
+__device__ __forceinline__ uint32_t run_word(uint32_t at, uint32_t step) { return at | step << 26; }
+
+// The slots of a node's 3^NDIM neighbour cells, in the order z, y, x: a row of three cells along x
+// lies in at most two blocks, so a row hashes at most two.
+template <int NDIM>
+struct Neighbours {
+  int hx, hy, hz;
+  uint32_t mask, seed;
+  uint32_t hyz;            // the hash of the row's block so far
+  uint32_t w;              // the row's place in its block
+  template <bool BATCH = false>  // the graph's seed is xored to the block's z, the plain one added
+  __device__ __forceinline__ void row(int dy, int dz) {
+    const int cy = hy + dy, cz = hz + dz;
+    if (NDIM == 3) {
+      const uint32_t bz = (uint32_t)cz >> 2;
+      hyz = fl::mix32((uint32_t)cy >> 2 ^ fl::mix32(BATCH ? bz ^ seed : bz + seed));
+      w = spread3_3(cy & 3) << 1 | spread3_3(cz & 3) << 2;
+    } else if (NDIM == 2) {
+      hyz = fl::mix32((uint32_t)cy >> 3 ^ fl::mix32(seed));
+      w = spread2_3(cy & 7) << 1;
+    } else {
+      hyz = fl::mix32(fl::mix32(seed));
+      w = 0;
+    }
+  }
+  __device__ __forceinline__ uint32_t slot(int dx) const {
+    const int cx = hx + dx;
+    const uint32_t bx = (uint32_t)cx >> (NDIM == 3 ? 2 : NDIM == 2 ? 3 : 6);
+    const uint32_t wx = NDIM == 3 ? spread3_3(cx & 3) : NDIM == 2 ? spread2_3(cx & 7) : (uint32_t)cx & 63u;
+    return ((fl::mix32(bx ^ hyz) << 6) + (wx | w)) & mask;
+  }
+};
+
+// Bound by the latency of the table's and the nodes' loads, which land all over L2: a node looks at
+// 27 cells, of which a sparse layout fills one in five. With one entry loaded after the other, a
+// check of the keys before and at each start and a list of the slots seen, the query of 100,000
+// nodes in 3D took 64 us, of 200,000 in 2D 30 us; now 22 and 21 (ncu).
+// Visits the sorted nodes of a node's neighbour cells, in the order of the cells and, in a cell, of the
+// sort: push(t, node t's record). KEY_SHIFT: the sorted keys' shift to a slot. The table's words of a
+// whole plane of cells are loaded before the first is looked at, and a row's first nodes with the
+// keys that confirm them, so that the loads overlap.
+template <int NDIM, bool BATCH, typename Push>
+__device__ __forceinline__ void visit_cells(Neighbours<NDIM> cells, const uint64_t* __restrict__ skeys,
+                                            const uint2* __restrict__ runs,
+                                            const float4* __restrict__ sorted, int n, int key_shift,
+                                            uint32_t step, Push push) {
+  constexpr int ROWS = NDIM > 1 ? 3 : 1, PLANES = NDIM > 2 ? 3 : 1;
+  for (int p = 0; p < PLANES; ++p) {
+    uint32_t slot[3 * ROWS];
+    uint2 run[3 * ROWS];
+#pragma unroll
+    for (int y = 0; y < ROWS; ++y) {
+      cells.template row<BATCH>(ROWS == 3 ? y - 1 : 0, PLANES == 3 ? p - 1 : 0);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) slot[3 * y + k] = cells.slot(k - 1), run[3 * y + k] = runs[slot[3 * y + k]];
+    }
+#pragma unroll
+    for (int y = 0; y < ROWS; ++y) {
+      bool ok[3];
+      float4 o[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const uint32_t start = run[3 * y + k].x & kRunMask;
+        ok[k] = !((run[3 * y + k].x ^ step << 26) >> 26) && start < (uint32_t)n;
+        if (ok[k]) {
+          o[k] = sorted[start];
+          ok[k] = skeys[start] == (uint64_t)slot[3 * y + k] << key_shift;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (!ok[k]) continue;
+        const uint32_t end = min(run[3 * y + k].y & kRunMask, (uint32_t)n);
+        uint32_t t = run[3 * y + k].x & kRunMask;
+        for (;;) {
+          push(t, o[k]);
+          if (++t >= end) break;
+          o[k] = sorted[t];
+        }
+      }
+    }
+  }
+}
+
 __device__ __forceinline__ int cell_coord(float s, float inv) {
   return (int)fminf(fmaxf(floorf(s * inv), -1073741824.f), 1073741824.f);
 }
 
 constexpr int kKeyThreads = 1024;
+// the query's registers: 80 hold a plane's loads; 8 blocks (64) took 25 us for 22, 10 (48) 29
+constexpr int kQueryThreads = 128, kQueryBlocks = 6;
 
 __global__ void __launch_bounds__(kKeyThreads) k_grid_keys(const float4* __restrict__ pos,
                                                         const float4* __restrict__ vel, int n,
@@ -148,61 +243,52 @@ __global__ void __launch_bounds__(kKeyThreads) k_grid_keys(const float4* __restr
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
-// Run starts, and the sorted nodes' snapshot position and radius.
+// The slots' runs, and the sorted nodes' snapshot position and radius.
 __global__ void __launch_bounds__(kThreads) k_grid_begin(const uint64_t* __restrict__ skeys,
                                                          const uint32_t* __restrict__ perm,
                                                          const float4* __restrict__ pos,
                                                          const float4* __restrict__ vel,
                                                          const float* __restrict__ radius, int n,
-                                                         int bits, uint32_t* __restrict__ starts,
-                                                         float4* __restrict__ sorted) {
+                                                         int bits, uint2* __restrict__ runs,
+                                                         float4* __restrict__ sorted, uint32_t step,
+                                                         const FlTick* __restrict__ tk) {
+  if (tk) step = tk->step;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint64_t k = skeys[s];
-  if (s == 0 || skeys[s - 1] != k) starts[(uint32_t)(k >> (64 - bits))] = (uint32_t)s;
+  const uint32_t slot = (uint32_t)(k >> (64 - bits));
+  if (s == 0 || skeys[s - 1] != k) runs[slot].x = run_word((uint32_t)s, step);
+  if (s == n - 1 || skeys[s + 1] != k) runs[slot].y = run_word((uint32_t)s + 1u, step);
   const uint32_t i = perm[s];
   const float4 p = pos[i], v = vel[i];
   sorted[s] = make_float4(p.x + v.x, p.y + v.y, p.z + v.z, radius[i]);
 }
 
-__global__ void __launch_bounds__(kThreads) k_grid_query(
+template <int NDIM>
+__global__ void __launch_bounds__(kQueryThreads, kQueryBlocks) k_grid_query(
     const uint64_t* __restrict__ skeys, const uint32_t* __restrict__ perm,
-    const uint32_t* __restrict__ starts, const float4* __restrict__ sorted,
-    const float4* __restrict__ vel_in, float4* __restrict__ vel_out, int n, int ndim, int bits,
-    float inv, float strength, uint32_t step, uint32_t seed, const FlTick* __restrict__ tk) {
+    const uint2* __restrict__ runs, const float4* __restrict__ sorted,
+    const float4* __restrict__ vel_in, float4* __restrict__ vel_out, int n, int bits, float inv,
+    float strength, uint32_t step, uint32_t seed, const FlTick* __restrict__ tk) {
   if (tk) step = tk->step, seed = tk->seed;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const float4 me4 = sorted[s];
   const uint32_t i = perm[s];
   const float3 me = make_float3(me4.x, me4.y, me4.z);
-  const float ri = me4.w, ri2 = ri * ri;
-  const uint32_t mask = (1u << bits) - 1;
-  const int hx = cell_coord(me.x, inv), hy = ndim > 1 ? cell_coord(me.y, inv) : 0,
-            hz = ndim > 2 ? cell_coord(me.z, inv) : 0;
-  const int ry = ndim > 1 ? 1 : 0, rz = ndim > 2 ? 1 : 0;
-  uint32_t seen[27];
-  int nseen = 0;
+  const float ri = me4.w;
+  Neighbours<NDIM> cells;
+  cells.hx = cell_coord(me.x, inv), cells.hy = NDIM > 1 ? cell_coord(me.y, inv) : 0;
+  cells.hz = NDIM > 2 ? cell_coord(me.z, inv) : 0;
+  cells.mask = (1u << bits) - 1, cells.seed = 0x9e3779b9u;
   float3 acc = make_float3(0.f, 0.f, 0.f);
-  for (int dz = -rz; dz <= rz; ++dz)
-    for (int dy = -ry; dy <= ry; ++dy)
-      for (int dx = -1; dx <= 1; ++dx) {
-        const uint32_t slot = cell_slot(hx + dx, hy + dy, hz + dz, ndim, mask);
-        bool again = false;
-        for (int q = 0; q < nseen; ++q) again |= seen[q] == slot;
-        if (again) continue;
-        seen[nseen++] = slot;
-        const uint32_t start = starts[slot];
-        const uint64_t key = (uint64_t)slot << (64 - bits);
-        if (start >= (uint32_t)n || skeys[start] != key || (start > 0 && skeys[start - 1] == key))
-          continue;
-        for (uint32_t t = start; t < (uint32_t)n && skeys[t] == key; ++t)
-          if (t != (uint32_t)s) pair_push(me, ri2, ri, sorted[t], i, perm[t], ndim, strength, step, seed, acc);
-      }
+  visit_cells<NDIM, false>(cells, skeys, runs, sorted, n, 64 - bits, step, [&](uint32_t t, float4 o) {
+    if (t != (uint32_t)s) pair_push(me, ri, o, i, perm, t, 0u, NDIM, strength, step, seed, acc);
+  });
   float4 v = vel_in[i];
   v.x += acc.x;
-  if (ndim > 1) v.y += acc.y;
-  if (ndim > 2) v.z += acc.z;
+  if (NDIM > 1) v.y += acc.y;
+  if (NDIM > 2) v.z += acc.z;
   vel_out[i] = v;
 }
 
@@ -270,17 +356,20 @@ __global__ void __launch_bounds__(kKeyThreads) k_bgrid_keys(
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
-// Run starts of the cells, and each sorted node's snapshot position, radius and graph.
+// The slots' runs, and each sorted node's snapshot position, radius and graph.
 __global__ void __launch_bounds__(kThreads) k_bgrid_begin(
     const uint64_t* __restrict__ skeys, const uint32_t* __restrict__ perm,
     const float4* __restrict__ pos, const float4* __restrict__ vel,
     const float* __restrict__ radius, const uint32_t* __restrict__ gid, int n, int bits,
-    uint32_t* __restrict__ starts, float4* __restrict__ sorted, uint32_t* __restrict__ sgid) {
+    uint2* __restrict__ runs, float4* __restrict__ sorted, uint32_t* __restrict__ sgid,
+    const FlTick* __restrict__ tk) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint64_t k = skeys[s];
   if (k == ~0ull) return;  // not taking part (and sorted after every node that does)
-  if (s == 0 || skeys[s - 1] != k) starts[(uint32_t)(k >> (63 - bits))] = (uint32_t)s;
+  const uint32_t slot = (uint32_t)(k >> (63 - bits));
+  if (s == 0 || skeys[s - 1] != k) runs[slot].x = run_word((uint32_t)s, tk->step);
+  if (s == n - 1 || skeys[s + 1] != k) runs[slot].y = run_word((uint32_t)s + 1u, tk->step);
   const uint32_t i = perm[s];
   const float4 p = pos[i], v = vel[i];
   sorted[s] = make_float4(p.x + v.x, p.y + v.y, p.z + v.z, radius[i]);
@@ -289,11 +378,12 @@ __global__ void __launch_bounds__(kThreads) k_bgrid_begin(
 
 // Each node's pushes from the overlapping nodes of its own graph in the 3^d cells around its
 // own (the jiggle's ids and step are the graph's own: the same alone or in any batch).
-__global__ void __launch_bounds__(kThreads) k_bgrid_query(
+template <int NDIM>
+__global__ void __launch_bounds__(kQueryThreads, kQueryBlocks) k_bgrid_query(
     const uint64_t* __restrict__ skeys, const uint32_t* __restrict__ perm,
-    const uint32_t* __restrict__ starts, const float4* __restrict__ sorted,
+    const uint2* __restrict__ runs, const float4* __restrict__ sorted,
     const uint32_t* __restrict__ sgid, const FlGraph* __restrict__ gr,
-    const float4* __restrict__ vel_in, float4* __restrict__ vel_out, int n, int ndim, int bits,
+    const float4* __restrict__ vel_in, float4* __restrict__ vel_out, int n, int bits,
     const FlTick* __restrict__ tk) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
@@ -306,34 +396,19 @@ __global__ void __launch_bounds__(kThreads) k_bgrid_query(
     const uint32_t first = (uint32_t)G.first, step = tk->step + G.tick0, seed = tk->seed;
     const float4 me4 = sorted[s];
     const float3 me = make_float3(me4.x, me4.y, me4.z);
-    const float ri = me4.w, ri2 = ri * ri;
-    const uint32_t mask = (1u << bits) - 1;
-    const int hx = cell_coord(me.x, G.cinv), hy = ndim > 1 ? cell_coord(me.y, G.cinv) : 0,
-              hz = ndim > 2 ? cell_coord(me.z, G.cinv) : 0;
-    const int ry = ndim > 1 ? 1 : 0, rz = ndim > 2 ? 1 : 0;
-    uint32_t seen[27];
-    int nseen = 0;
+    const float ri = me4.w, cinv = G.cinv, cstr = G.cstr;
+    Neighbours<NDIM> cells;
+    cells.hx = cell_coord(me.x, cinv), cells.hy = NDIM > 1 ? cell_coord(me.y, cinv) : 0;
+    cells.hz = NDIM > 2 ? cell_coord(me.z, cinv) : 0;
+    cells.mask = (1u << bits) - 1, cells.seed = fl::mix32(g + 0x9e3779b9u);
     float3 acc = make_float3(0.f, 0.f, 0.f);
-    for (int dz = -rz; dz <= rz; ++dz)
-      for (int dy = -ry; dy <= ry; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const uint32_t slot = bcell_slot(hx + dx, hy + dy, hz + dz, ndim, mask, g);
-          bool again = false;
-          for (int q = 0; q < nseen; ++q) again |= seen[q] == slot;
-          if (again) continue;
-          seen[nseen++] = slot;
-          const uint32_t start = starts[slot];
-          const uint64_t key = (uint64_t)slot << (63 - bits);
-          if (start >= (uint32_t)n || skeys[start] != key || (start > 0 && skeys[start - 1] == key))
-            continue;
-          for (uint32_t t = start; t < (uint32_t)n && skeys[t] == key; ++t)
-            if (t != (uint32_t)s && sgid[t] == g)
-              pair_push(me, ri2, ri, sorted[t], i - first, perm[t] - first, ndim, G.cstr, step,
-                        seed, acc);
-        }
+    visit_cells<NDIM, true>(cells, skeys, runs, sorted, n, 63 - bits, tk->step, [&](uint32_t t, float4 o) {
+      if (t != (uint32_t)s && sgid[t] == g)
+        pair_push(me, ri, o, i - first, perm, t, first, NDIM, cstr, step, seed, acc);
+    });
     v.x += acc.x;
-    if (ndim > 1) v.y += acc.y;
-    if (ndim > 2) v.z += acc.z;
+    if (NDIM > 1) v.y += acc.y;
+    if (NDIM > 2) v.z += acc.z;
   }
   vel_out[i] = v;
 }
@@ -358,9 +433,10 @@ void fl_launch_bgrid_query(const FlGridBufs* g, const uint64_t* skeys, const uin
                            int64_t* launches) {
   const int n = g->n, blocks = (n + kThreads - 1) / kThreads;
   k_bgrid_begin<<<blocks, kThreads, 0, st>>>(skeys, perm, pos, vel_in, radius, gid, n, g->bits,
-                                             g->starts, g->sorted, sgid);
-  k_bgrid_query<<<blocks, kThreads, 0, st>>>(skeys, perm, g->starts, g->sorted, sgid, gr, vel_in,
-                                             vel_out, n, ndim, g->bits, tk);
+                                             g->runs, g->sorted, sgid, tk);
+  auto* query = ndim == 3 ? k_bgrid_query<3> : ndim == 2 ? k_bgrid_query<2> : k_bgrid_query<1>;
+  query<<<(n + kQueryThreads - 1) / kQueryThreads, kQueryThreads, 0, st>>>(skeys, perm, g->runs, g->sorted, sgid, gr, vel_in, vel_out, n,
+                                     g->bits, tk);
   *launches += 2;
 }
 
@@ -378,7 +454,7 @@ void fl_launch_collide_allpairs(const float4* pos, const float4* vel_in, float4*
 size_t fl_grid_bytes(int64_t n) {
   int bits = 8;
   while ((int64_t(1) << bits) < 2 * n) ++bits;
-  return align256(4 * ((size_t)1 << bits)) + align256(16 * (size_t)(n > 0 ? n : 1));
+  return align256(8 * ((size_t)1 << bits)) + align256(16 * (size_t)(n > 0 ? n : 1));
 }
 
 void fl_grid_carve(FlGridBufs* g, void* base, int64_t n) {
@@ -386,7 +462,7 @@ void fl_grid_carve(FlGridBufs* g, void* base, int64_t n) {
   while ((int64_t(1) << bits) < 2 * n) ++bits;
   char* p = static_cast<char*>(base);
   g->n = (int)n, g->bits = bits;
-  g->starts = (uint32_t*)p, p += align256(4 * ((size_t)1 << bits));
+  g->runs = (uint2*)p, p += align256(8 * ((size_t)1 << bits));
   g->sorted = (float4*)p;
 }
 
@@ -406,9 +482,10 @@ void fl_launch_grid_query(const FlGridBufs* g, const uint64_t* skeys, const uint
                           uint32_t step, uint32_t seed, cudaStream_t st, int64_t* launches,
                           const FlTick* tk) {
   const int n = g->n, blocks = (n + kThreads - 1) / kThreads;
-  k_grid_begin<<<blocks, kThreads, 0, st>>>(skeys, perm, pos, vel_in, radius, n, g->bits, g->starts,
-                                            g->sorted);
-  k_grid_query<<<blocks, kThreads, 0, st>>>(skeys, perm, g->starts, g->sorted, vel_in, vel_out, n,
-                                            ndim, g->bits, inv_cell, strength, step, seed, tk);
+  k_grid_begin<<<blocks, kThreads, 0, st>>>(skeys, perm, pos, vel_in, radius, n, g->bits, g->runs,
+                                            g->sorted, step, tk);
+  auto* query = ndim == 3 ? k_grid_query<3> : ndim == 2 ? k_grid_query<2> : k_grid_query<1>;
+  query<<<(n + kQueryThreads - 1) / kQueryThreads, kQueryThreads, 0, st>>>(skeys, perm, g->runs, g->sorted, vel_in, vel_out, n, g->bits,
+                                     inv_cell, strength, step, seed, tk);
   *launches += 2;
 }

@@ -268,7 +268,7 @@ void fl_launch_collide_allpairs(const float4* pos, const float4* vel_in, float4*
                                 const FlTick* tk = nullptr);
 struct FlGridBufs {
   int n, bits;
-  uint32_t* starts;   // [2^bits] run start per slot (validated against the sorted keys)
+  uint2* runs;        // [2^bits] start and end of each slot's run, tagged with the tick
   float4* sorted;     // [n] sorted snapshot position, radius
 };
 size_t fl_grid_bytes(int64_t n);
