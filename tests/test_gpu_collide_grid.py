@@ -78,3 +78,23 @@ def test_words_of_earlier_ticks_are_not_trusted(dims, iterations):
     e.close(), fresh.close()
     np.testing.assert_array_equal(a[0], b[0])
     np.testing.assert_array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("dims", [1, 2, 3])
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 33, 511, 512, 513, 1025, 8191])
+def test_every_pair_of_a_small_layout(dims, n):
+    """The pass over all pairs (below 8,192 nodes) at the edges of its blocks of 8 nodes and tiles of
+    512, with the grid test's reference and tolerance."""
+    rng = np.random.default_rng(n * 4 + dims)
+    pos4 = np.zeros((n, 4), np.float32)
+    pos4[:, :dims] = rng.normal(5, 2.0 * n ** (1 / dims), (n, dims))
+    radii = rng.uniform(0.0, 4, n).astype(np.float32)
+    radii[::11] = 0.0
+    e = engine(pos4, None, dims, radii)
+    e.enqueue(np.array([1.0]), 1.0)
+    _, vel = e.sync()
+    e.close()
+    want = host(pos4[:, :dims].astype(np.float64), radii.astype(np.float64), 0.7)
+    known = np.isfinite(want).all(1)
+    assert np.isfinite(vel).all()
+    np.testing.assert_allclose(vel[known, :dims], want[known], rtol=2e-4, atol=2e-4)
