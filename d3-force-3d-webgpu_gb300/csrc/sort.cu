@@ -383,8 +383,9 @@ int64_t tiles_for(int64_t n) {
 }
 // the most tiles a sort of up to cap pairs has
 int64_t tiles_cap_for(int64_t cap) {
+  const int64_t small = (cap + 256 * kSortItemsMin - 1) / (256 * kSortItemsMin);
   const int64_t t = (cap + kSortTileMid - 1) / kSortTileMid;
-  return t > kSortTilesSmall ? t : kSortTilesSmall;
+  return t > kSortTilesSmall ? t : small < kSortTilesSmall ? small : kSortTilesSmall;
 }
 
 // True the first time it is called on the current device for `done` (a kernel's shared-memory
