@@ -388,8 +388,9 @@ def radix_sort_noalloc(keys_ptr, vals_ptr, n, lo_bit, keys_out_ptr, vals_out_ptr
         raise FlError(rc, (L.fl_last_error(None) or b"").decode())
 
 
-def desc_from_gpu(g, key, n):
-    """fl_force_desc from a force.gpu() dict (the reference's descriptor, src/*.js gpu()).
+def desc_from_gpu(g, key, n, arrays=True):
+    """fl_force_desc from a force.gpu() dict (the reference's descriptor, src/*.js gpu()); without
+    `arrays` the scalars only, for a force whose arrays of this version the engine holds.
 
     Returns (ForceDesc, keepalive arrays). Per-node arrays become float32 with non-numbers as 0,
     as the reference's floats() does (src/gpu/passes/util.js:17-22)."""
@@ -403,6 +404,8 @@ def desc_from_gpu(g, key, n):
     keep = []
 
     def f32(values, count):
+        if not arrays:
+            return None
         a = np.zeros(count, np.float32)
         if values is not None and count:
             v = np.asarray(values, dtype=np.float64)[:count]
@@ -417,7 +420,9 @@ def desc_from_gpu(g, key, n):
         d.distance_max2 = float(g["distanceMax2"])
         d.theta2 = float(g["theta2"])
     elif t == "link":
-        if "source" in g:  # arrays of endpoint indices instead of link objects
+        if not arrays:
+            m = len(g["source"] if "source" in g else g["links"])
+        elif "source" in g:  # arrays of endpoint indices instead of link objects
             src = np.ascontiguousarray(g["source"], dtype=np.int32)
             dst = np.ascontiguousarray(g["target"], dtype=np.int32)
             m = len(src)
@@ -426,11 +431,12 @@ def desc_from_gpu(g, key, n):
             m = len(links)
             src = np.fromiter((l["source"]["index"] for l in links), np.int32, count=m)
             dst = np.fromiter((l["target"]["index"] for l in links), np.int32, count=m)
-        if not m:
-            src = dst = np.zeros(1, np.int32)
-        keep += [src, dst]
         d.m = m
-        d.source, d.target = src.ctypes.data, dst.ctypes.data
+        if arrays:
+            if not m:
+                src = dst = np.zeros(1, np.int32)
+            keep += [src, dst]
+            d.source, d.target = src.ctypes.data, dst.ctypes.data
         d.link_distance = f32(g["distances"], m)
         d.link_strength = f32(g["strengths"], m)
         d.link_bias = f32(g["bias"], m)

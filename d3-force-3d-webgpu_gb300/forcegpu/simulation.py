@@ -59,6 +59,20 @@ def _num(v):
     return 0.0 if v != v else v
 
 
+_PLAIN = {float, int, np.float64, np.float32}
+
+
+def _column(nodes, key):
+    """_num(node.get(key)) of every node, as float64: in one conversion where every node has a plain
+    number (the common case: 60 us for 1,000 nodes, where a call per node takes 200), else one by one."""
+    values = [node.get(key) for node in nodes]
+    if _PLAIN.issuperset(map(type, values)):
+        a = np.array(values, np.float64)
+        a[np.isnan(a)] = 0.0
+        return a
+    return np.array([_num(v) for v in values], np.float64)
+
+
 def _nan(v):
     return v is None or (isinstance(v, float) and math.isnan(v))
 
@@ -73,6 +87,7 @@ class _NodeMirror:
         self.n = 0
         self.nDim = 2
         self.plan = []
+        self.sent = {}  # the forces whose arrays the engine holds, by id: (force, type, version)
         self.enqueued = 0
         self.landed = 0
         self.stale = False
@@ -82,38 +97,24 @@ class _NodeMirror:
 
     # --- JS -> GPU (src/gpu/engine.js:115-194) ---
     def _read(self, a, b):
-        nd = self.nDim
+        nodes = self.nodes[a:b]
         pos = np.zeros((b - a, 4), np.float64)
         fix = np.zeros((b - a, 4), np.float64)
         mask = np.zeros(b - a, np.uint8)
-        for k, node in enumerate(self.nodes[a:b]):
-            pos[k, 0] = _num(node.get("x"))
-            if nd > 1:
-                pos[k, 1] = _num(node.get("y"))
-            if nd > 2:
-                pos[k, 2] = _num(node.get("z"))
-            m = 0
-            if node.get("fx") is not None:
-                m |= 1
-                fix[k, 0] = float(node["fx"])
-            if nd > 1 and node.get("fy") is not None:
-                m |= 2
-                fix[k, 1] = float(node["fy"])
-            if nd > 2 and node.get("fz") is not None:
-                m |= 4
-                fix[k, 2] = float(node["fz"])
-            mask[k] = m
+        for k, axis in enumerate("xyz"[:self.nDim]):
+            pos[:len(nodes), k] = _column(nodes, axis)
+            pins = [node.get("f" + axis) for node in nodes]
+            if pins.count(None) < len(pins):
+                for i, pin in enumerate(pins):
+                    if pin is not None:
+                        mask[i] |= 1 << k
+                        fix[i, k] = float(pin)
         return pos, fix, mask
 
     def _read_vel(self):
-        nd = self.nDim
         vel = np.zeros((self.n, 4), np.float64)
-        for k, node in enumerate(self.nodes):
-            vel[k, 0] = _num(node.get("vx"))
-            if nd > 1:
-                vel[k, 1] = _num(node.get("vy"))
-            if nd > 2:
-                vel[k, 2] = _num(node.get("vz"))
+        for k, axis in enumerate("xyz"[:self.nDim]):
+            vel[:len(self.nodes), k] = _column(self.nodes, "v" + axis)
         return vel
 
     def upload_all(self, first=False):
@@ -158,39 +159,46 @@ class _NodeMirror:
 
     # --- GPU -> JS (src/gpu/engine.js:198-239) ---
     def land(self, pos, vel):
-        nd = self.nDim
-        for i, node in enumerate(self.nodes):
-            x = _num(node.get("x"))
-            y = _num(node.get("y")) if nd > 1 else 0.0
-            z = _num(node.get("z")) if nd > 2 else 0.0
-            s = self.shadow[i]
-            if x == s[0] and y == s[1] and z == s[2]:  # untouched since the last exchange
-                node["x"] = s[0] = float(pos[i, 0])
-                if nd > 1:
-                    node["y"] = s[1] = float(pos[i, 1])
-                if nd > 2:
-                    node["z"] = s[2] = float(pos[i, 2])
-            node["vx"] = float(vel[i, 0])
-            if nd > 1:
-                node["vy"] = float(vel[i, 1])
-            if nd > 2:
-                node["vz"] = float(vel[i, 2])
+        nodes, axes = self.nodes, "xyz"[:self.nDim]
+        m = len(nodes)
+        if m > self.n:
+            raise IndexError("%d nodes, but the simulation was given %d" % (m, self.n))
+        at = np.asarray(pos[:m, :self.nDim], np.float64)
+        untouched = np.ones(m, bool)  # since the last exchange
+        for k, axis in enumerate(axes):
+            untouched &= _column(nodes, axis) == self.shadow[:m, k]
+        self.shadow[:m, :self.nDim][untouched] = at[untouched]
+        mine = nodes if untouched.all() else [node for node, u in zip(nodes, untouched.tolist()) if u]
+        for k, axis in enumerate(axes):
+            for node, x in zip(mine, at[untouched, k].tolist()):
+                node[axis] = x
+            speed = "v" + axis
+            for node, v in zip(nodes, vel[:m, k].tolist()):
+                node[speed] = v
 
     # --- engine calls ---
     def set_nodes(self, nodes, nDim):
         self.nodes, self.n, self.nDim = nodes, len(nodes), nDim
         self.enqueued = self.landed = 0
-        self.plan = []
+        self.plan, self.sent = [], {}
         self.upload_all(first=True)
 
     def set_forces(self, forces):
-        descs = []
+        # the engine reads a force's arrays only when its version changes: those it holds are not
+        # converted again (1,000 nodes and 1,500 links: 1.1 ms)
+        sent, self.sent = self.sent, {}
+        unique = len({id(f) for f in forces}) == len(forces)
+        descs, held = [], {}
         for f in forces:
             if not callable(getattr(f, "gpu", None)):
                 raise FlError(FL_E_UNSUPPORTED, "force %r has no gpu() description" % (f,))
-            descs.append(desc_from_gpu(f.gpu() or {"type": None}, id(f), self.n))
+            g = f.gpu() or {"type": None}
+            state = (f, g.get("type"), g.get("version", 0))
+            known = unique and id(f) in sent and sent[id(f)][0] is f and sent[id(f)][1:] == state[1:]
+            descs.append(desc_from_gpu(g, id(f), self.n, arrays=not known))
+            held[id(f)] = state
         self.eng.set_forces(descs)
-        self.plan = list(forces)
+        self.plan, self.sent = list(forces), held
 
     def enqueue(self, alphas, decay):
         if not self.n:
