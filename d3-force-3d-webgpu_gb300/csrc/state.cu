@@ -100,13 +100,15 @@ __device__ void flush_partial(const Partial& q, int ndim, int want_box, int want
 }
 
 // Per-graph bounding boxes and position sums of a batch. Nodes are grouped by graph, so graph
-// ids do not decrease along the nodes: a block takes kBreduceItems * kThreads consecutive nodes;
-// in each of its warps every run of equal ids is reduced toward its first lane (shuffles that
-// stop at the run's end), which adds the run to the block's table of the graphs it covers
-// (shared-memory atomics); the table then goes to the graphs' records with one global atomic
-// per graph, axis and quantity. A run whose graph falls past the table (a block over many tiny
-// graphs) goes to its record directly.
-constexpr int kBreduceItems = 8, kBreduceSlots = 16;
+// ids do not decrease along the nodes: a warp takes 32 kBreduceItems consecutive nodes, and where
+// they belong to a few graphs (nearly everywhere), each lane sums its own nodes of a graph and the
+// lanes' sums are added once. Otherwise, node by node of the lanes, every run of equal ids is reduced
+// toward its first lane (shuffles that stop at the run's end). Either adds its sum to the block's
+// table of the graphs it covers (shared-memory atomics); the table then goes to the graphs' records
+// with one global atomic per graph, axis and quantity. A run whose graph falls past the table (a
+// block over many tiny graphs) goes to its record directly. Bound by the 128-bit integer arithmetic
+// (53 % of the ALU): 22 us for 1.05M nodes in 256 graphs, 74 when every 32 nodes were reduced apart.
+constexpr int kBreduceItems = 4, kBreduceSlots = 16, kBreduceGraphs = 4;
 __global__ void __launch_bounds__(kThreads) k_breduce(const float4* __restrict__ pos, int n,
                                                       int ndim, const uint32_t* __restrict__ gid,
                                                       FlReduce* red) {
@@ -121,33 +123,13 @@ __global__ void __launch_bounds__(kThreads) k_breduce(const float4* __restrict__
   }
   for (int i = threadIdx.x; i < kBreduceSlots; i += kThreads) s_bad[i] = 0u;
   __syncthreads();
-  for (int it = 0; it < kBreduceItems; ++it) {
-    const int64_t i = first + (int64_t)it * kThreads + threadIdx.x;
-    const bool ok = i < n;
-    const uint32_t g = ok ? gid[i] : 0xffffffffu;
-    float4 p = ok ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    uint32_t bad = 0;
-    float lo[3] = {p.x, p.y, p.z}, hi[3] = {p.x, p.y, p.z};
-    __int128 sm[3] = {fl::fx128(p.x, bad), ndim > 1 ? fl::fx128(p.y, bad) : 0,
-                      ndim > 2 ? fl::fx128(p.z, bad) : 0};
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t go = __shfl_down_sync(FL_FULL, g, o);
-      const bool same = lane + o < 32 && go == g;
-      const uint32_t bo = __shfl_down_sync(FL_FULL, bad, o);
-      if (same) bad += bo;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float a = __shfl_down_sync(FL_FULL, lo[k], o), b = __shfl_down_sync(FL_FULL, hi[k], o);
-        const __int128 c = fl::shfl_down128(sm[k], o);
-        if (same) lo[k] = fminf(lo[k], a), hi[k] = fmaxf(hi[k], b), sm[k] += c;
-      }
-    }
-    const uint32_t gp = __shfl_up_sync(FL_FULL, g, 1);
-    if (!ok || (lane > 0 && gp == g)) continue;  // not the first lane of its run
+  // a lane's box and sums of graph g, into the block's table or the graph's record
+  auto put = [&](uint32_t g, const float* lo, const float* hi, const __int128* sm, uint32_t bad) {
     const uint32_t slot = g - g0;
     if (slot < (uint32_t)kBreduceSlots) {
-      for (int k = 0; k < ndim; ++k) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (k >= ndim) break;
         atomicMax(&s_lo[slot][k], ~fl::ordered(lo[k]));
         atomicMax(&s_hi[slot][k], fl::ordered(hi[k]));
         fl::atomic_add128(&s_slo[slot][k], &s_shi[slot][k], sm[k]);
@@ -155,12 +137,64 @@ __global__ void __launch_bounds__(kThreads) k_breduce(const float4* __restrict__
       if (bad) atomicAdd(&s_bad[slot], bad);
     } else {
       FlReduce* r = red + g;
-      for (int k = 0; k < ndim; ++k) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (k >= ndim) break;
         atomicMax(&r->lo[k], ~fl::ordered(lo[k]));
         atomicMax(&r->hi[k], fl::ordered(hi[k]));
         fl::atomic_add128(&r->sum_lo[k], &r->sum_hi[k], sm[k]);
       }
       if (bad) atomicAdd(&r->bad, bad);
+    }
+  };
+  const int64_t wfirst = first + (int64_t)(threadIdx.x >> 5) * 32 * kBreduceItems;
+  const int64_t wend = wfirst + 32 * kBreduceItems < n ? wfirst + 32 * kBreduceItems : (int64_t)n;
+  const uint32_t ga = wfirst < n ? gid[wfirst] : 0u, gb = wfirst < n ? gid[wend - 1] : 0u;
+  if (gb - ga < (uint32_t)kBreduceGraphs) {  // warp-uniform
+    for (uint32_t g = ga; g <= gb && wfirst < n; ++g) {
+      Partial q;
+      bool any = false;
+#pragma unroll
+      for (int it = 0; it < kBreduceItems; ++it) {
+        const int64_t i = wfirst + 32 * it + lane;
+        if (i < wend && (ga == gb || gid[i] == g)) any = true, q.add(pos[i], ndim, 1);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          q.lo[k] = fminf(q.lo[k], __shfl_xor_sync(FL_FULL, q.lo[k], o));
+          q.hi[k] = fmaxf(q.hi[k], __shfl_xor_sync(FL_FULL, q.hi[k], o));
+          if (k < ndim) q.s[k] += fl::shfl_xor128(q.s[k], o);
+        }
+      q.bad = __reduce_add_sync(FL_FULL, q.bad);
+      if (__any_sync(FL_FULL, any) && lane == 0) put(g, q.lo, q.hi, q.s, q.bad);  // (a graph may be empty)
+    }
+  } else {
+    for (int it = 0; it < kBreduceItems; ++it) {
+      const int64_t i = wfirst + 32 * it + lane;
+      const bool ok = i < n;
+      const uint32_t g = ok ? gid[i] : 0xffffffffu;
+      float4 p = ok ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      uint32_t bad = 0;
+      float lo[3] = {p.x, p.y, p.z}, hi[3] = {p.x, p.y, p.z};
+      __int128 sm[3] = {fl::fx128(p.x, bad), ndim > 1 ? fl::fx128(p.y, bad) : 0,
+                        ndim > 2 ? fl::fx128(p.z, bad) : 0};
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t go = __shfl_down_sync(FL_FULL, g, o);
+        const bool same = lane + o < 32 && go == g;
+        const uint32_t bo = __shfl_down_sync(FL_FULL, bad, o);
+        if (same) bad += bo;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float a = __shfl_down_sync(FL_FULL, lo[k], o), b = __shfl_down_sync(FL_FULL, hi[k], o);
+          const __int128 c = fl::shfl_down128(sm[k], o);
+          if (same) lo[k] = fminf(lo[k], a), hi[k] = fmaxf(hi[k], b), sm[k] += c;
+        }
+      }
+      const uint32_t gp = __shfl_up_sync(FL_FULL, g, 1);
+      if (ok && (lane == 0 || gp != g)) put(g, lo, hi, sm, bad);  // the first lane of its run
     }
   }
   __syncthreads();

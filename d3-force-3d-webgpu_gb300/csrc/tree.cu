@@ -2057,8 +2057,9 @@ void fl_launch_allpairs(const float4* pos, const float* strength, float4* vel, i
 
 void fl_launch_bgraph(int graphs, int ndim, const int32_t* off, const FlReduce* red,
                       const FlBatchParams* prm, const double* alpha, FlGraph* gr, cudaStream_t st) {
-  k_bgraph<<<(graphs + kThreads - 1) / kThreads, kThreads, 0, st>>>(graphs, ndim, off, red, prm,
-                                                                    alpha, gr);
+  // one warp a block: the covers are FP64, a warp instruction of which holds its SM's pipe for 16
+  // clocks, so the warps want an SM each (256 graphs in one block took 14 us)
+  k_bgraph<<<(graphs + 31) / 32, 32, 0, st>>>(graphs, ndim, off, red, prm, alpha, gr);
 }
 
 void fl_launch_bmorton(const float4* pos, int n, int ndim, const uint32_t* gid, const FlGraph* gr,
