@@ -1376,7 +1376,9 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks) k_walk(
 // pushes the child's children. Each lane sums what it applied, and the warp adds the lanes'
 // sums in a fixed shuffle tree, so a layout is the same run after run. The stack holds the
 // bound on its depth in shared memory, 8 bytes an entry (first child slot; count | top depth
-// << 26), so nothing spills and the grid is not limited by spill regions.
+// << 26), so nothing spills and the grid is not limited by spill regions. Bound by instruction issue
+// (68 % of the slots): 20,000 points take some 9 rounds of 165 instructions each, 44 us; finding each
+// child's entry by marks in shared memory and a running maximum in place of one ballot took 47.
 // stats (STATS): [0] children tested, [1] of those, the ones the point's d3 traversal needs
 // (not a zero value, not the point itself; the union walk's [1], [3] and [4] count the same
 // (point, child) pairs), [2] deepest stack, [3] cells opened, [4] cells or points applied,
@@ -1392,7 +1394,6 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
   // at most 32 children per round and one push per child: the union walk's bound with G = 32
   constexpr int kAll = kWalkStackLayers(NDIM) * 32;
   __shared__ uint2 s_stack[kWalkWarps][kAll];
-  __shared__ uint32_t s_own[kWalkWarps][32];
   __shared__ float s_T0;
   if (threadIdx.x == 0) s_T0 = (float)((double)cube[3] * (double)cube[3] / theta2);
   __syncthreads();
@@ -1404,7 +1405,6 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
   unsigned long long st_tests = 0, st_useful = 0, st_open = 0, st_apply = 0, st_rare = 0;
   int maxsp = 0;
   uint2* stk = s_stack[warp];
-  uint32_t* sown = s_own[warp];
   int t = lane == 0 ? (int)atomicAdd(work, 1u) : 0;
   t = __shfl_sync(FL_FULL, t, 0);
   while (t < n) {
@@ -1417,48 +1417,30 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
     const uint32_t guard_max = 4u * (uint32_t)n + 64u;
     __syncwarp();
     while (sp > 0) {
-      // lane i reads the i-th entry from the top; a prefix sum of the entries' child counts
-      // places each entry's children in the round, and lane j finds the entry of child j
+      // the gather of the union walk: lane i reads the i-th entry from the top, a prefix sum of the
+      // entries' child counts places their children, lane j takes child j of the round
       const bool has = lane < sp;
       const uint2 se = has ? stk[sp - 1 - lane] : make_uint2(0u, 0u);
-      uint4 e = make_uint4(se.x, se.y & kCountMask, se.y >> 26, 0u);
-      if (has && (e.x >= slot_cap || e.y > slot_cap - e.x)) {  // a malformed tree: never read past it
+      uint32_t ex = se.x, ey = se.y & kCountMask;
+      if (has && (ex >= slot_cap || ey - 1u >= slot_cap - ex)) {  // a malformed tree: never read past it
         atomicOr(err, FL_ERR_TREE);
-        e.y = e.x >= slot_cap ? 0u : slot_cap - e.x;
+        ex = 0u, ey = 1u;
       }
-      uint32_t inc = e.y;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(FL_FULL, inc, o);
-        if (lane >= o) inc += u;
-      }
-      const uint32_t exc = inc - e.y;
-      const uint32_t avail = __shfl_sync(FL_FULL, inc, 31);
-      const uint32_t total = avail < 32u ? avail : 32u;
+      const uint32_t inc = inclusive_sum(ey), exc = inc - ey;
+      const uint32_t avail = __shfl_sync(FL_FULL, inc, 31), total = min(avail, 32u);
       // entries taken whole leave the stack; one taken in part keeps the rest (the new top)
       const uint32_t taken = __ballot_sync(FL_FULL, has && inc <= total);
-      if (has && exc < total && inc > total)
-        stk[sp - 1 - lane] = make_uint2(e.x + (total - exc), (inc - total) | e.z << 26);
+      if (avail > 32u && has && exc < 32u && inc > 32u)
+        stk[sp - 1 - lane] = make_uint2(ex + (32u - exc), (inc - 32u) | (se.y & ~kCountMask));
       sp -= __popc(taken);
-      sown[lane] = 0u;
-      __syncwarp();
-      if (e.y && exc < total) sown[exc] = (uint32_t)lane;
-      __syncwarp();
-      uint32_t own = sown[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(FL_FULL, own, o);
-        if (lane >= o && u > own) own = u;
-      }
-      const uint32_t own_first = __shfl_sync(FL_FULL, e.x, (int)own);
-      const uint32_t own_exc = __shfl_sync(FL_FULL, exc, (int)own);
-      const uint32_t my_top = __shfl_sync(FL_FULL, e.z, (int)own);
-      __syncwarp();
+      const uint32_t starts = __reduce_or_sync(FL_FULL, has && exc < total ? 1u << exc : 0u);
+      const int own = __popc(starts & (below_me | (1u << lane))) - 1;
+      const uint32_t slot = __shfl_sync(FL_FULL, ex - exc, own) + (uint32_t)lane;
+      const uint32_t my_top = __shfl_sync(FL_FULL, se.y >> 26, own);
       bool o = false, a = false, rare = false, need = false;
       uint2 m = make_uint2(0u, 0u);
       uint32_t D = 0;
       if ((uint32_t)lane < total) {
-        const uint32_t slot = own_first + ((uint32_t)lane - own_exc);
         const float4 q = __ldg(cdata + slot);
         m = __ldg(cmeta + slot);
         const bool lf = m.y == kLeafMark;
