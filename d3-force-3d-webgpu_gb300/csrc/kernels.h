@@ -180,8 +180,7 @@ struct FlTreeBufs {
   uint8_t* depth;        // [n-1] d3 depth of each internal node's cell
   uint32_t* count;       // [n-1] children of a head (0 for other nodes)
   uint32_t* first;       // [n-1] first child slot of a head
-  uint32_t* flag;        // [n] mixed-sign recursion: arrivals of each head's child cells; [n-1] the start count
-  uint32_t* up_list;     // [n-1] mixed-sign recursion: the heads without child cells
+  uint32_t* flag;        // [n-1] mixed-sign recursion: arrivals of each head's child cells
   float4* cell;          // [n-1] head: centroid, value at its own depth
   float4* leaf;          // [n] sorted points: position, strength
   float4* child_data;    // [2n] slot: centroid or position, value at own depth / strength

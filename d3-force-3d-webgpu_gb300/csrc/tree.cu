@@ -652,8 +652,7 @@ __device__ __forceinline__ float4 closed_cell(uint32_t i, int ndim, float sign,
 // Whether internal node i heads a d3 cell, and how many d3 children that cell has (its occupied
 // octants; at the deepest level, where the keys are equal, its points); the counts' exclusive
 // prefix within the block (first[]) and the block's total (ctot[]), for the slots. CLOSED (strengths
-// of one sign): a head's cell from the prefix sums too (closed_cell), into cell[]. Otherwise the
-// heads without child cells (where the recursion starts) are listed in up_list[0, *up_count).
+// of one sign): a head's cell from the prefix sums too (closed_cell), into cell[].
 template <bool CLOSED>
 __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
                                                     const uint32_t* __restrict__ parent,
@@ -667,42 +666,24 @@ __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
                                                     const D4* __restrict__ Ptot,
                                                     const float4* __restrict__ leaf,
                                                     const float* __restrict__ cube, int fx_exp,
-                                                    float4* __restrict__ cell, FlSegs seg,
-                                                    uint32_t* __restrict__ up_list,
-                                                    uint32_t* __restrict__ up_count) {
+                                                    float4* __restrict__ cell, FlSegs seg) {
   __shared__ uint32_t s_warp[kThreads / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t c = 0;
-  bool start = false;
   if (i < n - 1) {
     const int D = depth[i];
     if (D != kGapDepth) {
       const uint32_t pa = parent[i];
       const bool head = pa == (uint32_t)i || depth[pa] < D;  // a graph's root, or a deeper cell
       if (head) {
-        if (D >= levels_of(ndim)) {
-          c = range[2 * i + 1] - range[2 * i] + 1;
-          start = true;
-        } else {
-          const uint32_t om = omask[i];
-          c = __popc(om & 0xffffu);
-          start = !(om >> 16);
-        }
+        if (D >= levels_of(ndim)) c = range[2 * i + 1] - range[2 * i] + 1;
+        else c = __popc(omask[i] & 0xffffu);
       }
     }
     count[i] = c;
     if (CLOSED && c)
       cell[i] = closed_cell((uint32_t)i, ndim, sign, range, depth, P, Ptot, leaf, cube, fx_exp, seg);
-  }
-  if (!CLOSED) {  // one atomic per warp
-    const uint32_t bal = __ballot_sync(FL_FULL, start);
-    if (bal) {
-      uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(up_count, (uint32_t)__popc(bal));
-      base = __shfl_sync(FL_FULL, base, 0);
-      if (start) up_list[base + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)i;
-    }
   }
   uint32_t x = c;
 #pragma unroll
@@ -720,14 +701,20 @@ __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
 
 // The recursion itself (strengths of both signs), over the d3 cells from the deepest up, reading
 // each head's children from its slots (k_slots has written the points and every slot's meta).
-// The heads without child cells (k_heads listed them) start, one per thread. A finished cell
-// writes itself into its slot among its parent's children and counts itself in at the parent;
-// the last of the parent's child cells to arrive (their octants are the high half of the
-// parent's octant mask) puts the parent on its block's queue in shared memory, and the block
-// works through the queue a round at a time, one head per thread, until it is empty. So the
-// chain of dependent steps is the d3 depth, and a round's heads sit on consecutive lanes: FP64
-// runs at 2 lanes per clock per SM, and a warp instruction costs its 16 clocks however few of
-// its lanes are active, so heads climbing alone on scattered lanes made this pass FP64-bound.
+// A warp owns kUpNodes consecutive binary nodes and starts with its heads without child cells. A
+// finished cell writes itself into its slot among its parent's children and counts itself in at the
+// parent; the last of the parent's child cells to arrive (their octants are the high half of the
+// parent's octant mask) puts the parent on its warp's queue in shared memory, and the warp works
+// through the queue a round at a time, one head per lane, until it is empty. The binary nodes of
+// a cell over the sorted points [a, b] lie in a .. b (its own is a or b), so a parent whose points
+// lie in the warp's range has all its cells there: they count in shared memory, ordered by the
+// rounds. Only the cells above count in global memory, by a device-wide acquire-release, which
+// waits for the stores before it to reach L2.
+// So the chain of dependent steps is the d3 depth, and a round's heads sit on consecutive lanes: FP64
+// runs at 2 lanes per clock per SM, and a warp instruction costs its 16 clocks however few of its
+// lanes are active. Bound by that and by the chain of loads, counts and rounds: 300,000 points took
+// 114 us with one list of starts, every count in global memory and rounds of whole blocks, and take
+// 94 (ncu); a tick alone 499 -> 476 us.
 // A head combines its children as accumulate() does (src/manyBody.js:42-71). With
 // fp64_depth > 0 every value is d3's FP64 number bit for bit: the children's values summed in
 // slot order, which is d3's octant order (z << 2 | y << 1 | x), a chain of one-child cells
@@ -739,10 +726,11 @@ __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
 // values, summed in FP64 above fp64_depth and in FP32 below. fp64_depth 0 runs all of it in
 // FP32 (values within 2^-20 of their children's |values| count as 0), for precision
 // comparisons.
-// Children whose slots are loaded together: 1 measured fastest at 1M nodes (48 registers, more
-// blocks resident; 2 and 4 children, 60 and 70 registers, were 6 and 20 us slower per tick).
+// Children whose slots are loaded together, and nodes per warp: with 8 and 256 the pass alone takes
+// 87 us, but 120 registers slow the tick beside others' (316 us for 312).
 constexpr int kUpBatch = 1;
 constexpr uint32_t kNoHead = 0xffffffffu;
+constexpr int kUpThreads = 128, kUpWarps = kUpThreads / 32, kUpNodes = 128;
 
 // One head of the recursion: combine its children into its cell, write the cell into its slot
 // and count it in at its parent. Returns the parent when this was its last child cell to
@@ -751,7 +739,8 @@ __device__ __forceinline__ uint32_t cells_up_one(
     uint32_t h, int n, int ndim, const uint32_t* __restrict__ head_of,
     const uint32_t* __restrict__ omask, const uint8_t* __restrict__ depth,
     const uint32_t* __restrict__ count, const uint32_t* __restrict__ first,
-    const uint32_t* __restrict__ ctot, uint32_t* __restrict__ arrive, float4* cdata,
+    const uint32_t* __restrict__ ctot, const uint32_t* __restrict__ range,
+    uint32_t* __restrict__ arrive, uint32_t* s_arrive, uint32_t lo, float4* cdata,
     const uint2* __restrict__ cmeta, double* slot64, int fp64_depth, double c1, uint32_t* err,
     const FlSegs& seg) {
   const uint32_t roots = seg.graphs ? (uint32_t)seg.graphs : 1u;
@@ -764,7 +753,11 @@ __device__ __forceinline__ uint32_t cells_up_one(
   const bool root = !(rec & 0x80000000u);
   const uint32_t p = rec & kCountMask, oct = (rec >> 27) & 15u;
   uint32_t pcnt = 0, pfirst = 0, ptot = 0, pmask = 0;
-  if (!root) pcnt = count[p], pfirst = first[p], ptot = ctot[p >> 8], pmask = omask[p];
+  uint2 prange = make_uint2(0u, 0u);
+  if (!root) {
+    pcnt = count[p], pfirst = first[p], ptot = ctot[p >> 8], pmask = omask[p];
+    prange = reinterpret_cast<const uint2*>(range)[p];
+  }
   if (fs + cnt > nslots) {  // a malformed tree
     atomicOr(err, FL_ERR_TREE);
     return kNoHead;
@@ -843,43 +836,55 @@ __device__ __forceinline__ uint32_t cells_up_one(
   }
   cdata[slot] = out;
   if (exact) slot64[slot] = val;
+  if (prange.x >= lo && prange.y < lo + kUpNodes)  // all its binary nodes are the warp's
+    return atomicAdd(&s_arrive[p - lo], 1u) + 1u == (uint32_t)__popc(pmask >> 16) ? p : kNoHead;
   // acquire-release: each arrival publishes its cell; the last sees all of them
   const uint32_t w = cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(arrive[p])
                          .fetch_add(1u, cuda::memory_order_acq_rel);
   return w + 1u == (uint32_t)__popc(pmask >> 16) ? p : kNoHead;
 }
 
-__global__ void __launch_bounds__(kThreads) k_cells_up(
+__global__ void __launch_bounds__(kUpThreads) k_cells_up(
     int n, int ndim, const uint32_t* __restrict__ head_of, const uint32_t* __restrict__ omask,
     const uint8_t* __restrict__ depth, const uint32_t* __restrict__ count,
     const uint32_t* __restrict__ first, const uint32_t* __restrict__ ctot,
-    uint32_t* __restrict__ arrive, float4* cdata, const uint2* __restrict__ cmeta,
-    double* slot64, int fp64_depth, double c1, uint32_t* err, FlSegs seg,
-    const uint32_t* __restrict__ up_list, const uint32_t* __restrict__ up_count) {
-  __shared__ uint32_t s_queue[kThreads];
-  __shared__ uint32_t s_len;
-  const uint32_t starts = min(*up_count, (uint32_t)(n - 1));
-  if (blockIdx.x * blockDim.x >= starts) return;  // the whole block
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t h = t < starts ? up_list[t] : kNoHead;
-  for (int round = 0;; ++round) {
-    if (threadIdx.x == 0) s_len = 0;
-    __syncthreads();
-    if (h != kNoHead) {
-      if (round > 64) {  // deeper than any d3 tree: a malformed tree
-        atomicOr(err, FL_ERR_TREE);
-      } else {
-        const uint32_t next = cells_up_one(h, n, ndim, head_of, omask, depth, count, first,
-                                           ctot, arrive, cdata, cmeta, slot64, fp64_depth, c1,
-                                           err, seg);
-        if (next != kNoHead) s_queue[atomicAdd(&s_len, 1u)] = next;
-      }
+    const uint32_t* __restrict__ range, uint32_t* __restrict__ arrive, float4* cdata,
+    const uint2* __restrict__ cmeta, double* slot64, int fp64_depth, double c1, uint32_t* err,
+    FlSegs seg) {
+  // per warp: this round's heads and the next one's, and the arrivals at its own cells
+  __shared__ uint32_t s_queue[kUpWarps][2][kUpNodes];
+  __shared__ uint32_t s_arrive[kUpWarps][kUpNodes];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t below_me = (1u << lane) - 1u;
+  const uint32_t lo = (blockIdx.x * kUpWarps + warp) * kUpNodes;
+  uint32_t len = 0;
+  for (uint32_t k = 0; k < kUpNodes; k += 32) {
+    const uint32_t i = lo + k + lane;
+    s_arrive[warp][k + lane] = 0u;
+    const bool start = i < (uint32_t)(n - 1) && count[i] && (depth[i] >= levels_of(ndim) || !(omask[i] >> 16));
+    const uint32_t b = __ballot_sync(FL_FULL, start);
+    if (start) s_queue[warp][0][len + __popc(b & below_me)] = i;
+    len += __popc(b);
+  }
+  for (int round = 0; len; ++round) {
+    if (round > 64) {  // deeper than any d3 tree: a malformed tree
+      if (lane == 0) atomicOr(err, FL_ERR_TREE);
+      return;
     }
-    __syncthreads();
-    const uint32_t len = s_len;
-    h = threadIdx.x < len ? s_queue[threadIdx.x] : kNoHead;
-    if (len == 0) return;  // block-uniform
-    __syncthreads();  // everyone has its head before the queue is reset
+    __syncwarp();
+    const uint32_t* now = s_queue[warp][round & 1];
+    uint32_t* later = s_queue[warp][~round & 1];
+    uint32_t more = 0;
+    for (uint32_t k = 0; k < len; k += 32) {
+      uint32_t next = kNoHead;
+      if (k + lane < len)
+        next = cells_up_one(now[k + lane], n, ndim, head_of, omask, depth, count, first, ctot, range, arrive,
+                            s_arrive[warp], lo, cdata, cmeta, slot64, fp64_depth, c1, err, seg);
+      const uint32_t b = __ballot_sync(FL_FULL, next != kNoHead);
+      if (next != kNoHead) later[more + __popc(b & below_me)] = next;
+      more += __popc(b);
+    }
+    len = more;
   }
 }
 
@@ -1711,7 +1716,7 @@ size_t fl_tree_bytes(int64_t n) {
   const size_t m = (size_t)(n > 1 ? n - 1 : 1), N = (size_t)(n > 0 ? n : 1);
   const size_t blocks = (N + kThreads - 1) / kThreads;
   return align256(4 * m) * 3 + align256(4 * N) + align256(8 * m) + align256(m) +
-         align256(4 * m) * 3 + align256(4 * (m + 1)) + align256(16 * m) + align256(16 * N) +
+         align256(4 * m) * 3 + align256(16 * m) + align256(16 * N) +
          align256(16 * (2 * N + 1)) +
          align256(8 * (2 * N + 1)) * 2 + align256(4 * blocks) + align256(32 * N) +
          align256(32 * blocks) + align256(4 * m) + align256(4 * (2 * N)) +
@@ -1749,8 +1754,7 @@ void fl_tree_carve(FlTreeBufs* t, void* base, int64_t n, int ndim) {
   t->depth = (uint8_t*)take(m);
   t->count = (uint32_t*)take(4 * m);
   t->first = (uint32_t*)take(4 * m);
-  t->flag = (uint32_t*)take(4 * (m + 1));
-  t->up_list = (uint32_t*)take(4 * m);
+  t->flag = (uint32_t*)take(4 * m);
   t->slot64 = (double*)take(8 * (2 * N + 1));
   t->cell = (float4*)take(16 * m);
   t->leaf = (float4*)take(16 * N);
@@ -1845,17 +1849,14 @@ void fl_launch_cells(const FlTreeBufs* t, bool closed, float sign, const float* 
   uint32_t* ctot = static_cast<uint32_t*>(t->scan_scratch);
   const D4* P = reinterpret_cast<const D4*>(t->wsum);
   const D4* Ptot = reinterpret_cast<const D4*>(t->wtiles);
-  // the recursion's start list and its count, and the arrival counts (zeroed)
-  uint32_t* up_count = t->flag + m;
-  if (!closed) cudaMemsetAsync(t->flag, 0, 4 * (size_t)(m + 1), st);
   if (closed)
     k_heads<true><<<g, kThreads, 0, st>>>(n, t->ndim, t->parent, t->range, t->depth, t->omask,
                                           t->count, t->first, ctot, sign, P, Ptot, t->leaf, cube,
-                                          fx_exp, t->cell, segs, t->up_list, up_count);
+                                          fx_exp, t->cell, segs);
   else
     k_heads<false><<<g, kThreads, 0, st>>>(n, t->ndim, t->parent, t->range, t->depth, t->omask,
                                            t->count, t->first, ctot, sign, P, Ptot, t->leaf, cube,
-                                           fx_exp, t->cell, segs, t->up_list, up_count);
+                                           fx_exp, t->cell, segs);
   k_top_u32<<<1, kTopThreads, 0, st>>>(ctot, g);
   *launches += 2;
   k_slots<<<g2, kThreads, 0, st>>>(n, t->ndim, t->head_of, t->omask, t->parent, t->range,
@@ -1866,9 +1867,11 @@ void fl_launch_cells(const FlTreeBufs* t, bool closed, float sign, const float* 
   if (!closed) {
     // d3's c = Math.sqrt(4 / 2^dims), correctly rounded as IEEE sqrt is on host and device
     const double c1 = std::sqrt(4.0 / (double)(1 << t->ndim));
-    k_cells_up<<<g, kThreads, 0, st>>>(n, t->ndim, t->head_of, t->omask, t->depth, t->count,
-                                       t->first, ctot, t->flag, t->child_data, t->child_meta,
-                                       t->slot64, fp64_depth, c1, err, segs, t->up_list, up_count);
+    cudaMemsetAsync(t->flag, 0, 4 * (size_t)m, st);  // the arrivals
+    const int owned = kUpWarps * kUpNodes;
+    k_cells_up<<<(m + owned - 1) / owned, kUpThreads, 0, st>>>(
+        n, t->ndim, t->head_of, t->omask, t->depth, t->count, t->first, ctot, t->range, t->flag,
+        t->child_data, t->child_meta, t->slot64, fp64_depth, c1, err, segs);
     ++*launches;
   }
 }
