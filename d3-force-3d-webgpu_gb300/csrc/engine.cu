@@ -389,38 +389,37 @@ void encode_tree(fl_sim* s, Pass* p, const FlReduce* box, cudaStream_t st, FlRed
     ++s->launches;
     box = p->red.as<FlReduce>();
   }
-  // a small layout's keys are sorted in one launch (unless digit passes were asked for), so
-  // the keys need no digit histograms (lo_bit 64: none)
-  const bool by_rank = n <= kSortRankMax && s->sort_passes == 0;
+  // the closed form (exact fixed-point sums) when the strengths share one sign, unless a
+  // recursion was asked for
+  const bool closed = !p->mixed && s->cell_sums == FL_CELLS_AUTO;
+  const int fp64_depth = s->cell_sums == FL_CELLS_FP32 ? 0 : kRecursionFp64Depth;
+  if (n <= kSmallTreeMax && s->sort_passes == 0) {  // unless digit passes were asked for
+    Scope sc(s, G_BUILD, st);
+    fl_launch_small_tree(t, &p->sb, s->pos.as<float4>(), strength, box, zero, closed, p->sign,
+                         p->cube.as<float>(), p->fx_exp, fp64_depth, s->errw.as<uint32_t>(), st, &s->launches);
+    p->sorted_in = 1;
+    return;
+  }
   const int passes = (64 - lo_sort + 7) / 8;
   auto clean = [&](cudaStream_t cs) {  // what the next sort and the integrate want at zero
-    if (!by_rank) fl_sort_reset(&p->sb, n, passes, cs);
+    fl_sort_reset(&p->sb, n, passes, cs);
     if (zero) cudaMemsetAsync(zero, 0, sizeof(FlReduce), cs);
   };
   {
     Scope sc(s, G_MORTON, st);
     fl_launch_morton(s->pos.as<float4>(), n, s->ndim, box, p->sb.keys[0], p->sb.vals[0],
-                     by_rank ? nullptr : p->sb.hist, by_rank ? 64 : lo_sort, p->cube.as<float>(),
-                     st);
+                     p->sb.hist, lo_sort, p->cube.as<float>(), st);
     ++s->launches;
   }
   int r;
   {
     Scope sc(s, G_SORT, st);
-    if (by_rank) {
-      r = fl_sort_rank(&p->sb, n, st, &s->launches);
-    } else {
-      p->sb.test_spins = s->test_lookback;
-      r = fl_sort_passes(&p->sb, n, lo_sort, s->errw.as<uint32_t>(), st, &s->launches);
-      r = fl_sort_runfix(&p->sb, n, lo_bit, lo_sort, r, st, &s->launches);
-    }
+    p->sb.test_spins = s->test_lookback;
+    r = fl_sort_passes(&p->sb, n, lo_sort, s->errw.as<uint32_t>(), st, &s->launches);
+    r = fl_sort_runfix(&p->sb, n, lo_bit, lo_sort, r, st, &s->launches);
     p->sorted_in = r;
   }
   if (!(s->aux2 && !s->profiling)) clean(st);
-  // the closed form (exact fixed-point sums) when the strengths share one sign, unless a
-  // recursion was asked for
-  const bool closed = !p->mixed && s->cell_sums == FL_CELLS_AUTO;
-  const int fp64_depth = s->cell_sums == FL_CELLS_FP32 ? 0 : kRecursionFp64Depth;
   if (s->aux2 && !s->profiling) {
     // the internal nodes and the heads' octant masks on the third stream, beside the points
     cudaEventRecord(s->ev_fork2, st);

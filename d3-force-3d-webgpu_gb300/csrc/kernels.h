@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "common.cuh"
 
 // One tick's varying values, which the kernels read from device memory when given (null: the
@@ -116,12 +118,9 @@ int fl_sort_passes(const FlSortBufs* b, int64_t n, int lo_bit, uint32_t* err, cu
 int fl_sort_split(int lo_bit, int passes = 0);
 int fl_sort_runfix(const FlSortBufs* b, int64_t n, int lo_bit, int lo_sort, int cur,
                    cudaStream_t st, int64_t* launches);
-// Up to this many pairs, the tree sorts its keys in one launch (fl_sort_rank): each pair's place
-// counted against every key, the stable order of the digit passes and the run fix-up.
-constexpr int64_t kSortRankMax = 6144;
-// The stable sort of 1 <= n <= kSortRankMax pairs, keys[0]/vals[0] -> keys[1]/vals[1]; returns
-// the buffer holding the result (1), or 0 without a launch for other n.
-int fl_sort_rank(const FlSortBufs* b, int64_t n, cudaStream_t st, int64_t* launches);
+// True the first time it is called on the current device for `done` (a kernel's shared-memory
+// limit is raised once per device).
+bool fl_first_on_device(std::atomic<uint64_t>& done);
 
 // ---------------------------------------------------------------- state kernels (state.cu)
 void fl_launch_reduce(const float4* pos, int n, int ndim, int want_box, int want_sum,
@@ -231,6 +230,13 @@ void fl_launch_frontier(const FlTreeBufs* t, const uint64_t* skeys, uint32_t* er
 void fl_launch_cells(const FlTreeBufs* t, bool closed, float sign, const float* cube, int fx_exp,
                      int fp64_depth, uint32_t* err, cudaStream_t st, int64_t* launches,
                      FlSegs segs = {});
+// Up to this many points, one launch does the keys, their sort and all of the tree but the recursion
+// (from the bounding box `red`): the order of the digit passes and the run fix-up, the same tree. The
+// sorted pairs end in keys[1] / vals[1]; keys[0] and vals[0] are scratch. zero: a record to clear, or null.
+constexpr int kSmallTreeMax = 6144;
+void fl_launch_small_tree(const FlTreeBufs* t, const FlSortBufs* sb, const float4* pos, const float* strength,
+                          const FlReduce* red, FlReduce* zero, bool closed, float sign, float* cube, int fx_exp,
+                          int fp64_depth, uint32_t* err, cudaStream_t st, int64_t* launches);
 void fl_launch_build(const FlTreeBufs* t, const uint64_t* skeys, const uint32_t* perm,
                      const float4* pos, const float* strength, bool closed, const float* cube,
                      int fx_exp, cudaStream_t st, int64_t* launches, FlSegs segs = FlSegs{});

@@ -388,68 +388,19 @@ int64_t tiles_cap_for(int64_t cap) {
   return t > kSortTilesSmall ? t : small < kSortTilesSmall ? small : kSortTilesSmall;
 }
 
-// True the first time it is called on the current device for `done` (a kernel's shared-memory
-// limit is raised once per device, and on the first launch, which is never inside a capture).
-static bool first_on_device(std::atomic<uint64_t>& done) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return true;
-  const uint64_t bit = 1ull << dev;
-  return !(done.fetch_or(bit) & bit);
-}
-
 template <int T, int I>
 void launch_pass(const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout,
                  int64_t n, int shift, const uint32_t* ghist, uint32_t* status, uint32_t* ticket,
                  uint32_t* err, uint32_t spin_limit, int hold, cudaStream_t st) {
   static std::atomic<uint64_t> configured{0};
   const size_t dyn = (size_t)T * I * 12;
-  if (first_on_device(configured))
+  if (fl_first_on_device(configured))
     cudaFuncSetAttribute(k_onesweep<T, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
   const int64_t tiles = (n + T * I - 1) / (T * I);
   k_onesweep<T, I><<<(int)tiles, T, dyn, st>>>(kin, vin, kout, vout, n, shift, ghist, status,
                                                ticket, err, spin_limit, hold);
 }
 uint32_t longs_cap_for(int64_t n) { return (uint32_t)(n / (kRunShort + 1) + 1); }
-
-constexpr int kRankWarps = 8;
-
-// The stable sort of up to kSortRankMax pairs in one launch, for the tree of a small layout,
-// where the digit passes and the run fix-up are five launches over a few thousand keys. A pair's
-// place is the number of smaller keys plus the number of equal keys before it in the input.
-// Block b places pairs 32 b .. 32 b + 31: the block copies every key to shared memory
-// (coalesced), then lane l of every warp holds pair 32 b + l and counts over one kRankWarps-th
-// of the keys (the same key in every lane: a broadcast read); the warps' counts are summed in
-// shared memory.
-__global__ void __launch_bounds__(kRankWarps * 32) k_ranksort(const uint64_t* __restrict__ keys,
-                                                              const uint32_t* __restrict__ vals,
-                                                              int n, uint64_t* __restrict__ okeys,
-                                                              uint32_t* __restrict__ ovals) {
-  extern __shared__ uint64_t s_keys[];  // [n]
-  __shared__ uint32_t s_rank[kRankWarps][32];
-  for (int j = threadIdx.x; j < n; j += kRankWarps * 32) s_keys[j] = keys[j];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + lane;
-  const uint64_t k = i < n ? s_keys[i] : ~0ull;
-  const int per = (n + kRankWarps - 1) / kRankWarps;
-  const int j0 = min(n, w * per), j1 = min(n, j0 + per);
-  uint32_t rank = 0;
-#pragma unroll 8
-  for (int j = j0; j < j1; ++j) {
-    const uint64_t kj = s_keys[j];
-    rank += (uint32_t)((kj < k) | ((kj == k) & (j < i)));
-  }
-  s_rank[w][lane] = rank;
-  __syncthreads();
-  if (w == 0 && i < n) {
-    uint32_t r = 0;
-#pragma unroll
-    for (int q = 0; q < kRankWarps; ++q) r += s_rank[q][lane];
-    okeys[r] = k;
-    ovals[r] = vals[i];
-  }
-}
 
 }  // namespace
 
@@ -470,6 +421,14 @@ static FlSortShape sort_shape(int64_t n) {
   const int threads = n <= sms * 512 * kSortItems ? 512 : 1024;
   const int64_t it = (n + sms * threads - 1) / (sms * threads);
   return {threads, it < 5 ? 5 : (int)it};
+}
+
+bool fl_first_on_device(std::atomic<uint64_t>& done) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return true;
+  const uint64_t bit = 1ull << dev;
+  return !(done.fetch_or(bit) & bit);
 }
 
 int fl_sort_tile(int64_t n) {
@@ -570,18 +529,6 @@ int fl_sort_passes(const FlSortBufs* b, int64_t n, int lo_bit, uint32_t* err, cu
     cur = 1 - cur;
   }
   return cur;
-}
-
-int fl_sort_rank(const FlSortBufs* b, int64_t n, cudaStream_t st, int64_t* launches) {
-  if (n <= 0 || n > kSortRankMax) return 0;
-  static std::atomic<uint64_t> configured{0};
-  if (first_on_device(configured))
-    cudaFuncSetAttribute(k_ranksort, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(kSortRankMax * sizeof(uint64_t)));
-  k_ranksort<<<(int)((n + 31) / 32), kRankWarps * 32, (size_t)n * sizeof(uint64_t), st>>>(
-      b->keys[0], b->vals[0], (int)n, b->keys[1], b->vals[1]);
-  ++*launches;
-  return 1;
 }
 
 int fl_sort_split(int lo_bit, int passes) {

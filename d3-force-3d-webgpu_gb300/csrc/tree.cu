@@ -417,59 +417,28 @@ __device__ void block_prefix4(D4 v, D4* out, D4* tot, int i) {
   if (threadIdx.x == kThreads - 1) tot[blockIdx.x] = v;
 }
 
-// Karras (2012), "Maximizing parallelism in the construction of BVHs, octrees, and k-d trees":
-// internal node i covers sorted range [first, last] and splits it where the common prefix grows.
-// Thread i also gathers sorted point i and, for the closed-form cell sums, its record
-// (|a|, |a| u_x, |a| u_y, |a| u_z) with a = strength * c^leafDepth and u = (p - origin) / size in
-// [0, 1) the position in the d3 cube, as exact fixed point (scale 2^fx_exp, chosen so that no
-// sum over all points overflows), prefix-summed within the block. Integer sums are exact, and
-// cheap where FP64 is not.
-// PART: 1, the points (sorted leaves, records, their block prefix); 2, the internal nodes;
-// 0, both in one kernel.
-template <int PART>
-__global__ void __launch_bounds__(kThreads) k_build(
-    const uint64_t* __restrict__ k, const uint32_t* __restrict__ perm,
-    const float4* __restrict__ pos, const float* __restrict__ strength, int n, int ndim,
-    uint32_t* __restrict__ left, uint32_t* __restrict__ right, uint32_t* __restrict__ parent,
-    uint32_t* __restrict__ leaf_parent, uint32_t* __restrict__ range, uint8_t* __restrict__ depth,
-    float4* __restrict__ leaf, D4* __restrict__ wsum, D4* __restrict__ wtot,
-    const float* __restrict__ cube, int fx_exp, FlSegs seg) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// A sorted point's record for the closed-form cell sums: (|a|, |a| u_x, |a| u_y, |a| u_z) with
+// a = strength * c^leafDepth and u = (p - origin) / size in [0, 1) the position in the d3 cube, as
+// exact fixed point (scale 2^fe, chosen so that no sum over all points overflows). up, dn: the common
+// prefixes with the points after and before.
+__device__ __forceinline__ D4 point_record(float4 p, int up, int dn, int ndim, const float* cb, int fe) {
   const int L = levels_of(ndim), bits = L * ndim;
-  // the sorted range of this point's graph (a batch), and that graph's cube
-  int lo = 0, hi = n - 1;
-  const float* cb = cube;
-  int fe = fx_exp;
-  if (seg.graphs && i < n) {
-    const uint32_t g = seg.gid_pos[i];
-    lo = seg.off[g], hi = seg.off[g + 1] - 1;
-    cb = seg.g[g].origin;
-    fe = seg.g[g].fx;
-  }
-  const uint64_t ki = i < n ? k[i] : 0;
-  const int up = i < n ? kdelta(k, lo, hi, ki, i, i + 1) : -1;
-  const int dn = i < n ? kdelta(k, lo, hi, ki, i, i - 1) : -1;
-  if (PART != 2 && i < n && lo == hi) leaf_parent[i] = kNoParent;  // alone in its graph: no tree
-  D4 wrec = mk4(0, 0, 0, 0);
-  if (PART != 2 && i < n) {
-    const uint32_t node = perm[i];
-    float4 p = pos[node];
-    p.w = strength[node];
-    leaf[i] = p;
-    if (wsum) {
-      const int dmx = up > dn ? up : dn;
-      const int lD = (dmx >= bits ? L : dmx / ndim) + 1;  // the point's d3 leaf depth
-      const float sF = offset_scale(cb);
-      const long long W =
-          f2ll_rn(fabsf(p.w * damp(ndim, lD)) * __int_as_float((fe + 127) << 23));
-      wrec = mk4(W, mulhi62(W, fx_offset(p.x, cb[0], sF)),
-                 ndim > 1 ? mulhi62(W, fx_offset(p.y, cb[1], sF)) : 0,
-                 ndim > 2 ? mulhi62(W, fx_offset(p.z, cb[2], sF)) : 0);
-    }
-  }
-  if (PART != 2 && wsum)  // block-uniform
-    block_prefix4(wrec, wsum, wtot, i < n ? i : -1);
-  if (PART == 1 || i >= n - 1) return;
+  const int dmx = up > dn ? up : dn;
+  const int lD = (dmx >= bits ? L : dmx / ndim) + 1;  // the point's d3 leaf depth
+  const float sF = offset_scale(cb);
+  const long long W = f2ll_rn(fabsf(p.w * damp(ndim, lD)) * __int_as_float((fe + 127) << 23));
+  return mk4(W, mulhi62(W, fx_offset(p.x, cb[0], sF)), ndim > 1 ? mulhi62(W, fx_offset(p.y, cb[1], sF)) : 0,
+             ndim > 2 ? mulhi62(W, fx_offset(p.z, cb[2], sF)) : 0);
+}
+
+// Internal node i of the graph at sorted positions [lo, hi], lo < hi (i == hi: an index of no tree).
+// Karras (2012), "Maximizing parallelism in the construction of BVHs, octrees, and k-d trees": node i
+// covers a sorted range [first, last] and splits it where the common prefix grows.
+__device__ __forceinline__ void karras_node(const uint64_t* __restrict__ k, int lo, int hi, uint64_t ki,
+                                            int up, int dn, int i, int ndim, uint32_t* left,
+                                            uint32_t* right, uint32_t* parent, uint32_t* leaf_parent,
+                                            uint32_t* range, uint8_t* depth) {
+  const int L = levels_of(ndim), bits = L * ndim;
   if (i == hi) {  // the last point of a graph: this internal index belongs to no tree
     left[i] = right[i] = kNoParent;
     range[2 * i] = range[2 * i + 1] = (uint32_t)i;
@@ -505,11 +474,86 @@ __global__ void __launch_bounds__(kThreads) k_build(
   depth[i] = (uint8_t)(dep > L ? L : dep);
 }
 
+// The binary radix tree over the sorted keys (karras_node): thread i takes internal node i, gathers
+// sorted point i and, for the closed-form cell sums, its record (point_record), prefix-summed within
+// the block. Integer sums are exact, and cheap where FP64 is not.
+// PART: 1, the points (sorted leaves, records, their block prefix); 2, the internal nodes;
+// 0, both in one kernel.
+template <int PART>
+__global__ void __launch_bounds__(kThreads) k_build(
+    const uint64_t* __restrict__ k, const uint32_t* __restrict__ perm,
+    const float4* __restrict__ pos, const float* __restrict__ strength, int n, int ndim,
+    uint32_t* __restrict__ left, uint32_t* __restrict__ right, uint32_t* __restrict__ parent,
+    uint32_t* __restrict__ leaf_parent, uint32_t* __restrict__ range, uint8_t* __restrict__ depth,
+    uint32_t* __restrict__ omask, float4* __restrict__ leaf, D4* __restrict__ wsum, D4* __restrict__ wtot,
+    const float* __restrict__ cube, int fx_exp, FlSegs seg) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // the sorted range of this point's graph (a batch), and that graph's cube
+  int lo = 0, hi = n - 1;
+  const float* cb = cube;
+  int fe = fx_exp;
+  if (seg.graphs && i < n) {
+    const uint32_t g = seg.gid_pos[i];
+    lo = seg.off[g], hi = seg.off[g + 1] - 1;
+    cb = seg.g[g].origin;
+    fe = seg.g[g].fx;
+  }
+  const uint64_t ki = i < n ? k[i] : 0;
+  const int up = i < n ? kdelta(k, lo, hi, ki, i, i + 1) : -1;
+  const int dn = i < n ? kdelta(k, lo, hi, ki, i, i - 1) : -1;
+  if (PART != 2 && i < n && lo == hi) leaf_parent[i] = kNoParent;  // alone in its graph: no tree
+  D4 wrec = mk4(0, 0, 0, 0);
+  if (PART != 2 && i < n) {
+    const uint32_t node = perm[i];
+    float4 p = pos[node];
+    p.w = strength[node];
+    leaf[i] = p;
+    if (wsum) wrec = point_record(p, up, dn, ndim, cb, fe);
+  }
+  if (PART != 2 && wsum)  // block-uniform
+    block_prefix4(wrec, wsum, wtot, i < n ? i : -1);
+  if (PART == 1 || i >= n - 1) return;
+  omask[i] = 0u;  // k_frontier marks the octants
+  karras_node(k, lo, hi, ki, up, dn, i, ndim, left, right, parent, leaf_parent, range, depth);
+}
+
 // Every binary node below the root that is a d3 child (a point, or an internal node deeper than
 // its parent: the first node of another cell) finds the head of its parent's cell, climbing the
 // binary nodes of equal depth, and marks its octant (its keys' digit at the parent's depth) in
-// the head's octant mask. head_of[] keeps head | octant << 27 | 1 << 31 for the slots.
-// Threads [0, n-1) take the internal nodes, [n-1, 2n-1) the points (sorted order).
+// the head's octant mask. Returns head | octant << 27 | 1 << 31 for the slots, 0 for other nodes.
+// pt: x is a point (sorted order), else an internal node.
+__device__ __forceinline__ uint32_t frontier_of(bool pt, uint32_t x, int ndim, const uint64_t* skeys,
+                                                const uint32_t* parent, const uint32_t* leaf_parent,
+                                                const uint32_t* range, const uint8_t* depth,
+                                                uint32_t* omask, uint32_t* err) {
+  // the parent cell's binary node: none for a graph's root, an index between two graphs, or a
+  // point alone in its graph
+  uint32_t p = kNoParent;
+  if (pt) p = leaf_parent[x];
+  else if (depth[x] != kGapDepth && parent[x] != x) p = parent[x];
+  if (p == kNoParent) return 0u;
+  const int Dp = depth[p];
+  if (!pt && depth[x] <= Dp) return 0u;
+  uint32_t h = p;
+  for (int guard = 0;; ++guard) {  // equal depths: splits inside one cell
+    const uint32_t up = parent[h];
+    if (up == h || depth[up] < Dp) break;
+    h = up;
+    if (guard > 64) {
+      atomicOr(err, FL_ERR_TREE);
+      break;
+    }
+  }
+  uint32_t oct = 0;
+  if (Dp < levels_of(ndim)) {
+    const uint64_t k = skeys[pt ? x : range[2 * x]];
+    oct = (uint32_t)(k >> (64 - ndim * (Dp + 1))) & ((1u << ndim) - 1u);
+    atomicOr(omask + h, (1u << oct) | (pt ? 0u : 1u << (16 + oct)));  // cells also above
+  }
+  return h | (oct << 27) | 0x80000000u;
+}
+
+// Threads [0, n-1) take the internal nodes, [n-1, 2n-1) the points.
 __global__ void __launch_bounds__(kThreads) k_frontier(
     int n, int ndim, const uint64_t* __restrict__ skeys, const uint32_t* __restrict__ parent,
     const uint32_t* __restrict__ leaf_parent, const uint32_t* __restrict__ range,
@@ -518,38 +562,9 @@ __global__ void __launch_bounds__(kThreads) k_frontier(
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 2 * n - 1) return;
   const bool pt = t >= n - 1;
-  const uint32_t x = pt ? (uint32_t)(t - (n - 1)) : (uint32_t)t;
-  uint32_t rec = 0;
-  // the parent cell's binary node: none for a graph's root, an index between two graphs, or a
-  // point alone in its graph
-  uint32_t p = kNoParent;
-  if (pt) p = leaf_parent[x];
-  else if (depth[x] != kGapDepth && parent[x] != x) p = parent[x];
-  if (p != kNoParent) {
-    const int Dp = depth[p];
-    if (pt || depth[x] > Dp) {
-      uint32_t h = p;
-      for (int guard = 0;; ++guard) {  // equal depths: splits inside one cell
-        const uint32_t up = parent[h];
-        if (up == h || depth[up] < Dp) break;
-        h = up;
-        if (guard > 64) {
-          atomicOr(err, FL_ERR_TREE);
-          break;
-        }
-      }
-      uint32_t oct = 0;
-      if (Dp < levels_of(ndim)) {
-        const uint64_t k = skeys[pt ? x : range[2 * x]];
-        oct = (uint32_t)(k >> (64 - ndim * (Dp + 1))) & ((1u << ndim) - 1u);
-        atomicOr(omask + h, (1u << oct) | (pt ? 0u : 1u << (16 + oct)));  // cells also above
-      }
-      rec = h | (oct << 27) | 0x80000000u;
-    }
-  }
-  head_of[t] = rec;
+  head_of[t] = frontier_of(pt, pt ? (uint32_t)(t - (n - 1)) : (uint32_t)t, ndim, skeys, parent, leaf_parent,
+                           range, depth, omask, err);
 }
-
 
 // Exclusive prefix of the block totals, in place, by one block of kTopThreads: each thread sums
 // a run of consecutive totals, a warp-shuffle scan of the threads' sums (two levels) gives each
@@ -649,9 +664,19 @@ __device__ __forceinline__ float4 closed_cell(uint32_t i, int ndim, float sign,
   return out;
 }
 
-// Whether internal node i heads a d3 cell, and how many d3 children that cell has (its occupied
-// octants; at the deepest level, where the keys are equal, its points); the counts' exclusive
-// prefix within the block (first[]) and the block's total (ctot[]), for the slots. CLOSED (strengths
+// The d3 children of the cell that internal node i heads (its occupied octants; at the deepest level,
+// where the keys are equal, its points); 0 when i heads none.
+__device__ __forceinline__ uint32_t head_children(uint32_t i, int ndim, const uint32_t* parent,
+                                                  const uint32_t* range, const uint8_t* depth,
+                                                  const uint32_t* omask) {
+  const int D = depth[i];
+  if (D == kGapDepth) return 0u;
+  const uint32_t pa = parent[i];
+  if (!(pa == i || depth[pa] < D)) return 0u;  // a graph's root, or a deeper cell
+  return D >= levels_of(ndim) ? range[2 * i + 1] - range[2 * i] + 1 : (uint32_t)__popc(omask[i] & 0xffffu);
+}
+
+// Every head's count of children (head_children); the counts' exclusive prefix within the block (first[]) and the block's total (ctot[]), for the slots. CLOSED (strengths
 // of one sign): a head's cell from the prefix sums too (closed_cell), into cell[].
 template <bool CLOSED>
 __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
@@ -666,21 +691,15 @@ __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
                                                     const D4* __restrict__ Ptot,
                                                     const float4* __restrict__ leaf,
                                                     const float* __restrict__ cube, int fx_exp,
-                                                    float4* __restrict__ cell, FlSegs seg) {
+                                                    float4* __restrict__ cell,
+                                                    uint32_t* __restrict__ arrive, FlSegs seg) {
   __shared__ uint32_t s_warp[kThreads / 32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t c = 0;
   if (i < n - 1) {
-    const int D = depth[i];
-    if (D != kGapDepth) {
-      const uint32_t pa = parent[i];
-      const bool head = pa == (uint32_t)i || depth[pa] < D;  // a graph's root, or a deeper cell
-      if (head) {
-        if (D >= levels_of(ndim)) c = range[2 * i + 1] - range[2 * i] + 1;
-        else c = __popc(omask[i] & 0xffffu);
-      }
-    }
+    c = head_children((uint32_t)i, ndim, parent, range, depth, omask);
+    if (!CLOSED) arrive[i] = 0u;  // the recursion's arrivals
     count[i] = c;
     if (CLOSED && c)
       cell[i] = closed_cell((uint32_t)i, ndim, sign, range, depth, P, Ptot, leaf, cube, fx_exp, seg);
@@ -888,9 +907,38 @@ __global__ void __launch_bounds__(kUpThreads) k_cells_up(
   }
 }
 
-// Every d3 child writes itself into its slot of its head's cell: the head's first slot plus the
-// child's rank (occupied octants before its own; at the deepest level, its place in the range);
-// the root also fills slot 0. Threads as in k_frontier.
+// Child x (frontier record rec) writes itself into its slot of its head's cell: the head's first slot
+// plus the child's rank (occupied octants before its own; at the deepest level, its place in the
+// range). l: the point, or the cell (CELL: its own; else the recursion writes it later).
+template <bool CELL>
+__device__ __forceinline__ void write_slot(bool pt, uint32_t x, uint32_t rec, int n, int ndim, uint32_t roots,
+                                           const uint32_t* omask, const uint32_t* range,
+                                           const uint8_t* depth, const uint32_t* count,
+                                           const uint32_t* first, const uint32_t* ctot, const float4* l,
+                                           float4* cdata, uint2* cmeta, double* slot64, uint32_t* err) {
+  if (!(rec & 0x80000000u)) return;
+  const uint32_t h = rec & kCountMask, oct = (rec >> 27) & 15u;
+  const uint32_t rank = depth[h] >= levels_of(ndim)
+                            ? (pt ? x : range[2 * x]) - range[2 * h]
+                            : (uint32_t)__popc(omask[h] & ((1u << oct) - 1u));
+  const uint32_t slot = first_slot(first, ctot, h, roots) + rank;
+  if (rank >= count[h] || slot >= 2u * (uint32_t)n + 1u) {  // a malformed tree
+    atomicOr(err, FL_ERR_TREE);
+    return;
+  }
+  if (pt) {
+    const float4 p = *l;
+    cdata[slot] = p;
+    // the recursion's FP64 value of the point, converted here on full warps
+    if (slot64) slot64[slot] = (double)p.w;
+    cmeta[slot] = make_uint2(x, kLeafMark);
+  } else {
+    if (CELL) cdata[slot] = *l;
+    cmeta[slot] = make_uint2(first_slot(first, ctot, x, roots), count[x] | ((uint32_t)depth[x] << 26));
+  }
+}
+
+// Every d3 child into its slot; a root also fills its own. Threads as in k_frontier.
 __global__ void __launch_bounds__(kThreads) k_slots(
     int n, int ndim, const uint32_t* __restrict__ head_of, const uint32_t* __restrict__ omask,
     const uint32_t* __restrict__ parent,
@@ -910,25 +958,217 @@ __global__ void __launch_bounds__(kThreads) k_slots(
     cmeta[rs] = make_uint2(first_slot(first, ctot, x, roots), count[x] | ((uint32_t)depth[x] << 26));
   }
   const uint32_t rec = head_of[t];
-  if (!(rec & 0x80000000u)) return;
-  const uint32_t h = rec & kCountMask, oct = (rec >> 27) & 15u;
-  const uint32_t rank = depth[h] >= levels_of(ndim)
-                            ? (pt ? x : range[2 * x]) - range[2 * h]
-                            : (uint32_t)__popc(omask[h] & ((1u << oct) - 1u));
-  const uint32_t slot = first_slot(first, ctot, h, roots) + rank;
-  if (rank >= count[h] || slot >= 2u * (uint32_t)n + 1u) {  // a malformed tree
-    atomicOr(err, FL_ERR_TREE);
-    return;
+  const float4* l = pt ? leaf + x : cell + x;
+  if (cells_later)
+    write_slot<false>(pt, x, rec, n, ndim, roots, omask, range, depth, count, first, ctot, l, cdata, cmeta,
+                      slot64, err);
+  else
+    write_slot<true>(pt, x, rec, n, ndim, roots, omask, range, depth, count, first, ctot, l, cdata, cmeta,
+                     slot64, err);
+}
+
+// The whole tree of a layout of up to kSmallTreeMax points in one launch: one cluster of up to 8
+// blocks, a point per thread, a cluster barrier where the passes of a large layout are launches
+// (the bodies are theirs, and so are the arrays left in global memory). Blocks own kSmallRun * k
+// consecutive points (by input, then by sorted order).
+//   keys    each run of 256 sorted by a bitonic network (shuffles below a warp), the runs of a block
+//           merged by binary searches among each other, then the blocks' slices the same way: a
+//           pair's place is its place in its slice plus the pairs before it in the others (equal
+//           keys: those of earlier inputs, which keeps the order of a stable sort)
+//   nodes   Karras' searches on all the sorted keys in shared memory
+// The rest reads what other blocks wrote after a cluster barrier (release / acquire).
+// Bound by the chain of dependent steps, not by work: a launch, and an L2 round trip per pass. Against
+// eight launches and two memsets (the keys, a sort by counting, the tree's passes) a tick went from
+// 20.5 to 15.7 us at 1,000 points and from 44.9 to 35.2 at 5,000 (2D, with collide).
+constexpr int kSmallRun = 256, kSmallMaxThreads = 768, kSmallBlocks = 8;
+static_assert(kSmallTreeMax == kSmallMaxThreads * kSmallBlocks, "a point per thread");
+struct SmallTree {
+  const float4* pos;
+  const float* strength;
+  const FlReduce* red;
+  FlReduce* zero;  // a record to clear, or null
+  uint64_t *tmp, *keys;
+  uint32_t *vtmp, *perm;
+  float* cube;
+  uint32_t* err;
+  FlTreeBufs t;
+  float sign;
+  int fx_exp;
+  bool slots64;
+};
+
+// the keys among sorted a[0, len) before key: the smaller ones, and the equal ones with ties
+__device__ __forceinline__ uint32_t keys_before(const uint64_t* a, int len, uint64_t key, bool ties, int top) {
+  int at = 0;
+  for (int step = top; step; step >>= 1) {
+    const int q = at + step;
+    if (q <= len) {
+      const uint64_t o = a[q - 1];
+      if (o < key || (ties && o == key)) at = q;
+    }
   }
-  if (pt) {
-    const float4 l = leaf[x];
-    cdata[slot] = l;
-    // the recursion's FP64 value of the point, converted here on full warps
-    if (slot64) slot64[slot] = (double)l.w;
-    cmeta[slot] = make_uint2(x, kLeafMark);
-  } else {
-    if (!cells_later) cdata[slot] = cell[x];
-    cmeta[slot] = make_uint2(first_slot(first, ctot, x, roots), count[x] | ((uint32_t)depth[x] << 26));
+  return (uint32_t)at;
+}
+
+template <bool CLOSED>
+__global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree a) {
+  extern __shared__ uint64_t s_key[];  // [max(n, 1.5 slice)]: a slice's pairs in exchange, then all keys
+  __shared__ float s_cube[5];
+  __shared__ D4 s_warp4[kSmallMaxThreads / 32];
+  __shared__ uint32_t s_warp[kSmallMaxThreads / 32];
+  __shared__ D4 s_base4[kSmallTreeMax / 256];
+  __shared__ uint32_t s_base[kSmallTreeMax / 256];
+  namespace cg = cooperative_groups;
+  const int n = a.t.n, ndim = a.t.ndim, S = blockDim.x, C = gridDim.x, c = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i = c * S + tid;  // this thread's point, sorted point and internal node
+  const bool ok = i < n, node = i < n - 1;
+  const int used = (n + S - 1) / S;  // blocks with points
+  auto sync = [&] {
+    if (C > 1) cg::this_cluster().sync();
+    else __syncthreads();
+  };
+  const uint32_t idx0 = (uint32_t)i;
+  float4 p = ok ? a.pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid == 0) {
+    d3_cover(a.red, ndim, s_cube);
+    if (c == 0)
+      for (int k = 0; k < 5; ++k) a.cube[k] = s_cube[k];
+  }
+  if (a.zero && c == C - 1)
+    for (int k = tid; k < (int)(sizeof(FlReduce) / 4); k += S) reinterpret_cast<uint32_t*>(a.zero)[k] = 0u;
+  __syncthreads();
+  // ---- keys, sorted by (key, input)
+  uint64_t key = ok ? morton_key(p, s_cube, levels_of(ndim) - (int)s_cube[4], ndim) : ~0ull;
+  uint32_t idx = idx0;  // past the end: the largest key and input of all, so they end last
+  uint32_t* s_idx = reinterpret_cast<uint32_t*>(s_key + S);
+  const int r = tid & (kSmallRun - 1);
+  for (int k = 2; k <= kSmallRun; k <<= 1)
+    for (int j = k >> 1; j; j >>= 1) {
+      uint64_t ko;
+      uint32_t io;
+      if (j >= 32) {  // block-uniform
+        __syncthreads();
+        s_key[tid] = key, s_idx[tid] = idx;
+        __syncthreads();
+        ko = s_key[tid ^ j], io = s_idx[tid ^ j];
+      } else {
+        ko = __shfl_xor_sync(FL_FULL, key, j), io = __shfl_xor_sync(FL_FULL, idx, j);
+      }
+      const bool greater = key > ko || (key == ko && idx > io);
+      if (((r & j) == 0) == ((r & k) == 0) ? greater : !greater) key = ko, idx = io;
+    }
+  if (S > kSmallRun) {  // the block's runs into its slice's order
+    __syncthreads();
+    s_key[tid] = key;
+    __syncthreads();
+    uint32_t at = (uint32_t)r;
+    for (int q = 0; q < S; q += kSmallRun)
+      if (q != tid - r) at += keys_before(s_key + q, kSmallRun, key, q < tid - r, kSmallRun);
+    __syncthreads();
+    s_key[at] = key, s_idx[at] = idx;
+    __syncthreads();
+    key = s_key[tid], idx = s_idx[tid];
+  }
+  if (C > 1) {
+    if (ok) a.tmp[i] = key;
+    sync();
+    for (int j = tid; j < n; j += S) s_key[j] = a.tmp[j];
+    __syncthreads();
+  }
+  if (ok) {
+    uint32_t at = (uint32_t)tid;
+    for (int q = 0; q < used; ++q)
+      if (q != c)
+        at += keys_before(s_key + q * S, min(S, n - q * S), key, q < c, S >= 512 ? 512 : 256);
+    a.keys[at] = key;
+    a.perm[at] = idx;
+    p = a.pos[idx];
+    p.w = a.strength[idx];
+    a.t.leaf[at] = p;
+  }
+  sync();
+  for (int j = tid; j < n; j += S) s_key[j] = a.keys[j];
+  __syncthreads();
+  // ---- the binary tree, and the points' records
+  key = ok ? s_key[i] : 0;
+  const int up = ok ? kdelta(s_key, 0, n - 1, key, i, i + 1) : -1;
+  const int dn = ok ? kdelta(s_key, 0, n - 1, key, i, i - 1) : -1;
+  if (CLOSED) {
+    D4 v = mk4(0, 0, 0, 0);
+    if (ok) v = point_record(a.t.leaf[i], up, dn, ndim, s_cube, a.fx_exp);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const D4 y = shfl_up4(v, o);
+      if (lane >= o) v = add4(v, y);
+    }
+    if (lane == 31) s_warp4[warp] = v;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) v = add4(v, s_warp4[w]);
+    if (ok) reinterpret_cast<D4*>(a.t.wsum)[i] = v;
+    if (tid == S - 1 && c < used) reinterpret_cast<D4*>(a.t.wtiles)[c] = v;
+  }
+  if (node) {
+    a.t.omask[i] = 0u;
+    if (!CLOSED) a.t.flag[i] = 0u;
+    karras_node(s_key, 0, n - 1, key, up, dn, i, ndim, a.t.left, a.t.right, a.t.parent, a.t.leaf_parent,
+                a.t.range, a.t.depth);
+  }
+  sync();
+  // ---- the heads of the children's cells
+  const uint32_t nrec = node ? frontier_of(false, i, ndim, s_key, a.t.parent, a.t.leaf_parent, a.t.range,
+                                           a.t.depth, a.t.omask, a.err) : 0u;
+  const uint32_t prec = ok ? frontier_of(true, i, ndim, s_key, a.t.parent, a.t.leaf_parent, a.t.range,
+                                         a.t.depth, a.t.omask, a.err) : 0u;
+  if (!CLOSED && node) a.t.head_of[i] = nrec;
+  if (CLOSED && tid < (n + 255) / 256) {  // the records of the blocks before, per 256 points
+    D4 b = mk4(0, 0, 0, 0);
+    for (int q = 0; q < tid * 256 / S; ++q) b = add4(b, reinterpret_cast<const D4*>(a.t.wtiles)[q]);
+    s_base4[tid] = b;
+  }
+  sync();
+  // ---- the heads' children counted, their cells, and their first slots
+  uint32_t cnt = 0;
+  float4 cell = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (node) {
+    cnt = head_children((uint32_t)i, ndim, a.t.parent, a.t.range, a.t.depth, a.t.omask);
+    a.t.count[i] = cnt;
+    if (CLOSED && cnt)
+      cell = closed_cell((uint32_t)i, ndim, a.sign, a.t.range, a.t.depth,
+                         reinterpret_cast<const D4*>(a.t.wsum), s_base4, a.t.leaf, s_cube, a.fx_exp, FlSegs{});
+  }
+  uint32_t x = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FL_FULL, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_warp[warp] = x;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) x += s_warp[w];
+  if (node) a.t.first[i] = x - cnt;
+  if (tid == S - 1) a.vtmp[c] = x;  // the block's children
+  sync();
+  if (tid < (n + 255) / 256) {
+    uint32_t b = 0;
+    for (int q = 0; q < tid * 256 / S; ++q) b += a.vtmp[q];
+    s_base[tid] = b;
+    if (!CLOSED && c == 0) static_cast<uint32_t*>(a.t.scan_scratch)[tid] = b;
+  }
+  __syncthreads();
+  // ---- the slots
+  double* slot64 = a.slots64 ? a.t.slot64 : nullptr;
+  if (i == 0) {  // the root's own slot
+    if (CLOSED) a.t.child_data[0] = cell;
+    a.t.child_meta[0] = make_uint2(first_slot(a.t.first, s_base, 0u, 1u), cnt | ((uint32_t)a.t.depth[0] << 26));
+  }
+  if (node)
+    write_slot<CLOSED>(false, i, nrec, n, ndim, 1u, a.t.omask, a.t.range, a.t.depth, a.t.count, a.t.first,
+                       s_base, &cell, a.t.child_data, a.t.child_meta, slot64, a.err);
+  if (ok) {
+    const float4 l = a.t.leaf[i];
+    write_slot<CLOSED>(true, i, prec, n, ndim, 1u, a.t.omask, a.t.range, a.t.depth, a.t.count, a.t.first,
+                       s_base, &l, a.t.child_data, a.t.child_meta, slot64, a.err);
   }
 }
 
@@ -1801,7 +2041,7 @@ void fl_launch_build_points(const FlTreeBufs* t, const uint64_t* skeys, const ui
   const int n = t->n;
   const int nb = (n + kThreads - 1) / kThreads;
   k_build<1><<<nb, kThreads, 0, st>>>(skeys, perm, pos, strength, n, t->ndim, t->left, t->right,
-                                      t->parent, t->leaf_parent, t->range, t->depth, t->leaf,
+                                      t->parent, t->leaf_parent, t->range, t->depth, t->omask, t->leaf,
                                       closed ? reinterpret_cast<D4*>(t->wsum) : nullptr,
                                       reinterpret_cast<D4*>(t->wtiles), cube, fx_exp, segs);
   ++*launches;
@@ -1817,7 +2057,7 @@ void fl_launch_build_nodes(const FlTreeBufs* t, const uint64_t* skeys, const uin
   const int n = t->n;
   const int nb = (n + kThreads - 1) / kThreads;
   k_build<2><<<nb, kThreads, 0, st>>>(skeys, perm, pos, strength, n, t->ndim, t->left, t->right,
-                                      t->parent, t->leaf_parent, t->range, t->depth, t->leaf,
+                                      t->parent, t->leaf_parent, t->range, t->depth, t->omask, t->leaf,
                                       nullptr, nullptr, cube, fx_exp, segs);
   ++*launches;
 }
@@ -1833,12 +2073,56 @@ void fl_launch_build(const FlTreeBufs* t, const uint64_t* skeys, const uint32_t*
 
 void fl_launch_frontier(const FlTreeBufs* t, const uint64_t* skeys, uint32_t* err,
                         cudaStream_t st, int64_t* launches) {
-  const int n = t->n, m = n - 1;
+  const int n = t->n;
   const int g2 = (2 * n - 1 + kThreads - 1) / kThreads;
-  cudaMemsetAsync(t->omask, 0, 4 * (size_t)m, st);
   k_frontier<<<g2, kThreads, 0, st>>>(n, t->ndim, skeys, t->parent, t->leaf_parent, t->range,
                                       t->depth, t->omask, t->head_of, err);
   ++*launches;
+}
+
+// The recursion, once every slot has its meta and the arrivals are zero.
+static void launch_cells_up(const FlTreeBufs* t, int fp64_depth, uint32_t* err, cudaStream_t st,
+                            int64_t* launches, FlSegs segs) {
+  const int n = t->n, owned = kUpWarps * kUpNodes;
+  // d3's c = Math.sqrt(4 / 2^dims), correctly rounded as IEEE sqrt is on host and device
+  const double c1 = std::sqrt(4.0 / (double)(1 << t->ndim));
+  k_cells_up<<<(n - 1 + owned - 1) / owned, kUpThreads, 0, st>>>(
+      n, t->ndim, t->head_of, t->omask, t->depth, t->count, t->first,
+      static_cast<const uint32_t*>(t->scan_scratch), t->range, t->flag, t->child_data, t->child_meta,
+      t->slot64, fp64_depth, c1, err, segs);
+  ++*launches;
+}
+
+void fl_launch_small_tree(const FlTreeBufs* t, const FlSortBufs* sb, const float4* pos, const float* strength,
+                          const FlReduce* red, FlReduce* zero, bool closed, float sign, float* cube, int fx_exp,
+                          int fp64_depth, uint32_t* err, cudaStream_t st, int64_t* launches) {
+  const int n = t->n;
+  SmallTree a;
+  a.pos = pos, a.strength = strength, a.red = red, a.zero = zero;
+  a.tmp = sb->keys[0], a.keys = sb->keys[1], a.vtmp = sb->vals[0], a.perm = sb->vals[1];
+  a.cube = cube, a.err = err, a.t = *t, a.sign = sign, a.fx_exp = fx_exp;
+  a.slots64 = !closed && fp64_depth != 0;
+  static std::atomic<uint64_t> configured{0};
+  if (fl_first_on_device(configured)) {
+    cudaFuncSetAttribute(k_small_tree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kSmallTreeMax);
+    cudaFuncSetAttribute(k_small_tree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kSmallTreeMax);
+  }
+  const int slice = kSmallRun * ((n + kSmallRun * kSmallBlocks - 1) / (kSmallRun * kSmallBlocks));
+  int blocks = 1;
+  while (blocks * slice < n) blocks *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)slice);
+  cfg.dynamicSmemBytes = (size_t)(8 * n > 12 * slice ? 8 * n : 12 * slice);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)blocks, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr, cfg.numAttrs = blocks > 1 ? 1 : 0;
+  if (closed) cudaLaunchKernelEx(&cfg, k_small_tree<true>, a);
+  else cudaLaunchKernelEx(&cfg, k_small_tree<false>, a);
+  ++*launches;
+  if (!closed) launch_cells_up(t, fp64_depth, err, st, launches, FlSegs{});
 }
 
 void fl_launch_cells(const FlTreeBufs* t, bool closed, float sign, const float* cube, int fx_exp,
@@ -1852,11 +2136,11 @@ void fl_launch_cells(const FlTreeBufs* t, bool closed, float sign, const float* 
   if (closed)
     k_heads<true><<<g, kThreads, 0, st>>>(n, t->ndim, t->parent, t->range, t->depth, t->omask,
                                           t->count, t->first, ctot, sign, P, Ptot, t->leaf, cube,
-                                          fx_exp, t->cell, segs);
+                                          fx_exp, t->cell, t->flag, segs);
   else
     k_heads<false><<<g, kThreads, 0, st>>>(n, t->ndim, t->parent, t->range, t->depth, t->omask,
                                            t->count, t->first, ctot, sign, P, Ptot, t->leaf, cube,
-                                           fx_exp, t->cell, segs);
+                                           fx_exp, t->cell, t->flag, segs);
   k_top_u32<<<1, kTopThreads, 0, st>>>(ctot, g);
   *launches += 2;
   k_slots<<<g2, kThreads, 0, st>>>(n, t->ndim, t->head_of, t->omask, t->parent, t->range,
@@ -1864,16 +2148,7 @@ void fl_launch_cells(const FlTreeBufs* t, bool closed, float sign, const float* 
                                    t->child_data, t->child_meta, err, segs, !closed,
                                    closed || fp64_depth == 0 ? nullptr : t->slot64);
   ++*launches;
-  if (!closed) {
-    // d3's c = Math.sqrt(4 / 2^dims), correctly rounded as IEEE sqrt is on host and device
-    const double c1 = std::sqrt(4.0 / (double)(1 << t->ndim));
-    cudaMemsetAsync(t->flag, 0, 4 * (size_t)m, st);  // the arrivals
-    const int owned = kUpWarps * kUpNodes;
-    k_cells_up<<<(m + owned - 1) / owned, kUpThreads, 0, st>>>(
-        n, t->ndim, t->head_of, t->omask, t->depth, t->count, t->first, ctot, t->range, t->flag,
-        t->child_data, t->child_meta, t->slot64, fp64_depth, c1, err, segs);
-    ++*launches;
-  }
+  if (!closed) launch_cells_up(t, fp64_depth, err, st, launches, segs);
 }
 
 void fl_launch_aggregate(const FlTreeBufs* t, const uint64_t* skeys, bool closed, float sign,
