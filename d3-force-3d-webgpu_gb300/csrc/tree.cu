@@ -169,18 +169,31 @@ __device__ __forceinline__ uint64_t cell_of(float x, float origin, int e, uint32
 }
 
 // d3 cover() of a bounding box (d3-octree): origin = floor(min); a power-of-two size doubled
-// until max < origin + size (FP64, one thread). cube5 = origin x, y, z, size, log2 size.
+// until max < origin + size (FP64). cube5 = origin x, y, z, size, log2 size, written by lane 0; every
+// lane of the warp calls it, and tries a size of its own: one thread's chain of FP64 sums and
+// compares took 3,600 clocks for 11 doublings, at the start of every tick.
 __device__ void d3_cover(const FlReduce* red, int ndim, float* cube5) {
   double lo0 = 0, lo1 = 0, lo2 = 0, hi0 = 0, hi1 = 0, hi2 = 0;
   lo0 = floor((double)fl::unordered(~red->lo[0])), hi0 = (double)fl::unordered(red->hi[0]);
   if (ndim > 1) lo1 = floor((double)fl::unordered(~red->lo[1])), hi1 = (double)fl::unordered(red->hi[1]);
   if (ndim > 2) lo2 = floor((double)fl::unordered(~red->lo[2])), hi2 = (double)fl::unordered(red->hi[2]);
-  double size = 1;
-  int lg = 0;
-  while (lg < 1100 && !(hi0 < lo0 + size && (ndim < 2 || hi1 < lo1 + size) && (ndim < 3 || hi2 < lo2 + size)))
-    size *= 2, ++lg;
-  cube5[0] = (float)lo0, cube5[1] = (float)lo1, cube5[2] = (float)lo2;
-  cube5[3] = (float)size, cube5[4] = (float)lg;
+  // lane k tries the size 2^(base + k); past 2^1023 doubling gives infinity
+  const auto size_of = [](int k) { return k < 1024 ? __longlong_as_double((long long)(k + 1023) << 52) : (double)INFINITY; };
+  int lg = 1100;
+  for (int base = 0; base < 1100; base += 32) {
+    const int k = base + (int)fl::lane_id();
+    const double size = size_of(k);
+    const uint32_t fits = __ballot_sync(FL_FULL, k < 1100 && hi0 < lo0 + size && (ndim < 2 || hi1 < lo1 + size) &&
+                                                     (ndim < 3 || hi2 < lo2 + size));
+    if (fits) {
+      lg = base + __ffs(fits) - 1;
+      break;
+    }
+  }
+  if (fl::lane_id() == 0) {
+    cube5[0] = (float)lo0, cube5[1] = (float)lo1, cube5[2] = (float)lo2;
+    cube5[3] = (float)size_of(lg), cube5[4] = (float)lg;
+  }
 }
 
 // The left-aligned Morton key of p in the cube with the given origin, e = LEVELS - log2(size).
@@ -211,9 +224,9 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const float4* __restr
   __shared__ float s_cube[5];
   __shared__ uint32_t sh[8 * 256];
   const int passes = (64 - lo_bit + 7) / 8;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     d3_cover(red, ndim, s_cube);
-    if (blockIdx.x == 0)
+    if (blockIdx.x == 0 && threadIdx.x == 0)
       for (int k = 0; k < 5; ++k) cube_out[k] = s_cube[k];
   }
   for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) sh[i] = 0;
@@ -239,15 +252,15 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const float4* __restr
 
 // ---- batches of graphs: the per-graph tick values, the keys, and the sort by graph
 
-// One thread per graph: the graph's d3 cube from its bounding box, the walk's threshold, its
+// One warp per graph: the graph's d3 cube from its bounding box, the walk's threshold, its
 // distances, this tick's alpha, its velocity multiplier and its centre force's shift.
 __global__ void __launch_bounds__(kThreads) k_bgraph(int graphs, int ndim, const int32_t* __restrict__ off,
                                                      const FlReduce* __restrict__ red,
                                                      const FlBatchParams* __restrict__ prm,
                                                      const double* __restrict__ alpha,
                                                      FlGraph* __restrict__ gr) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= graphs) return;
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+  if (g >= graphs) return;  // the whole warp
   FlGraph o;
   const int first = off[g], count = off[g + 1] - off[g];
   if (count > 0) {
@@ -255,6 +268,7 @@ __global__ void __launch_bounds__(kThreads) k_bgraph(int graphs, int ndim, const
   } else {
     o.origin[0] = o.origin[1] = o.origin[2] = 0.f, o.size = 1.f, o.lg = 0.f;
   }
+  if (fl::lane_id()) return;
   const FlBatchParams p = prm[g];
   o.T0 = (float)((double)o.size * (double)o.size / p.theta2);
   o.dmin2 = (float)p.dmin2;
@@ -434,33 +448,74 @@ __device__ __forceinline__ D4 point_record(float4 p, int up, int dn, int ndim, c
 // Internal node i of the graph at sorted positions [lo, hi], lo < hi (i == hi: an index of no tree).
 // Karras (2012), "Maximizing parallelism in the construction of BVHs, octrees, and k-d trees": node i
 // covers a sorted range [first, last] and splits it where the common prefix grows.
-__device__ __forceinline__ void karras_node(const uint64_t* __restrict__ k, int lo, int hi, uint64_t ki,
-                                            int up, int dn, int i, int ndim, uint32_t* left,
-                                            uint32_t* right, uint32_t* parent, uint32_t* leaf_parent,
-                                            uint32_t* range, uint8_t* depth) {
+// Returns first, last and the d3 depth of the node's cell.
+// A search step asks whether a common prefix is longer than d bits: whether the keys' exclusive or is at
+// most its largest value then, a compare instead of a count of leading zeros.
+__device__ __forceinline__ uint64_t prefix_mask(int d) { return d < 63 ? ~0ull >> (d + 1) : 0ull; }
+// WIDE: 12 and then 7 probes at once, for a few warps an SM, which wait for each probe's latency: 5,300
+// clocks for 7,400 at 1,000 points (4 blocks of 256). With 24 warps an SM, or a chip full of them, the
+// probes' work counts and one at a time is faster (10,300 clocks for 11,600 at 5,000 points).
+template <bool WIDE>
+__device__ __forceinline__ uint3 karras_node(const uint64_t* __restrict__ k, int lo, int hi, uint64_t ki,
+                                             int up, int dn, int i, int ndim, uint32_t* left,
+                                             uint32_t* right, uint32_t* parent, uint32_t* leaf_parent,
+                                             uint32_t* range, uint8_t* depth) {
   const int L = levels_of(ndim), bits = L * ndim;
   if (i == hi) {  // the last point of a graph: this internal index belongs to no tree
     left[i] = right[i] = kNoParent;
     range[2 * i] = range[2 * i + 1] = (uint32_t)i;
     depth[i] = kGapDepth;
-    return;
+    return make_uint3((uint32_t)i, (uint32_t)i, (uint32_t)kGapDepth);
   }
   if (i == lo) parent[i] = (uint32_t)i;  // a graph's root is its own parent
   const int d = up > dn ? 1 : -1;
   const int dmin = up > dn ? dn : up;
-  int64_t lmax = 2;
-  while (kdelta(k, lo, hi, ki, i, (int)(i + lmax * d)) > dmin) lmax *= 2;
-  int64_t len = 0;
-  for (int64_t t = lmax >> 1; t >= 1; t >>= 1)
-    if (kdelta(k, lo, hi, ki, i, (int)(i + (len + t) * d)) > dmin) len += t;
-  const int j = (int)(i + len * d);
+  // whether the prefix of keys i and j is longer than `than` bits, m its mask (equal keys: the
+  // indices' bits follow)
+  const auto longer = [&](int j, int than, uint64_t m) {
+    if (WIDE) {  // read in any case: no branch to diverge at
+      const int in = min(max(j, lo), hi);
+      const uint64_t x = ki ^ k[in];
+      return (bool)((in == j) & (x <= m) & ((than < 64) | (64 + __clz(i ^ j) > than)));
+    }
+    if (j < lo || j > hi) return false;
+    const uint64_t x = ki ^ k[j];
+    return x <= m && (than < 64 || 64 + __clz(i ^ j) > than);
+  };
+  const uint64_t mmin = prefix_mask(dmin);
+  // the most l with longer(i + l d) (it falls as l grows, and holds for from): below from + w, w a
+  // power of two
+  const auto farthest = [&](int from, int w, int than, uint64_t m) {
+    int l = from;
+    if (WIDE) {
+      while (w > 1) {
+        const int q = w > 8 ? w >> 3 : 1;
+        int hits = 0;
+#pragma unroll
+        for (int e = 1; e < 8; ++e) hits += longer(i + (l + e * q) * d, than, m);
+        l += hits * q;
+        w = q;
+      }
+    } else {
+      for (int t = w >> 1; t >= 1; t >>= 1)
+        if (longer(i + (l + t) * d, than, m)) l += t;
+    }
+    return l;
+  };
+  int lmax = 1;  // below 2^28, as the indices are
+  if (WIDE) {
+    int hits = 0;
+#pragma unroll
+    for (int e = 1; e < 13; ++e) hits += longer(i + d * (1 << e), dmin, mmin);  // kSmallTreeMax < 2^13
+    lmax = 1 << hits;
+  } else {
+    while (longer(i + 2 * lmax * d, dmin, mmin)) lmax *= 2;
+  }
+  const int len = farthest(lmax, lmax, dmin, mmin);
+  const int j = i + len * d;
   const int dnode = kdelta(k, lo, hi, ki, i, j);
-  int64_t s = 0, t = len;
-  do {
-    t = (t + 1) >> 1;
-    if (kdelta(k, lo, hi, ki, i, (int)(i + (s + t) * d)) > dnode) s += t;
-  } while (t > 1);
-  const int split = (int)(i + s * d + (d < 0 ? -1 : 0));
+  const int s = farthest(0, 1 << (32 - __clz(len)), dnode, prefix_mask(dnode));
+  const int split = i + s * d + (d < 0 ? -1 : 0);
   const int first = i < j ? i : j, last = i < j ? j : i;
   uint32_t l = first == split ? (kLeaf | (uint32_t)split) : (uint32_t)split;
   uint32_t r = last == split + 1 ? (kLeaf | (uint32_t)(split + 1)) : (uint32_t)(split + 1);
@@ -471,7 +526,9 @@ __device__ __forceinline__ void karras_node(const uint64_t* __restrict__ k, int 
   else parent[r] = (uint32_t)i;
   range[2 * i] = (uint32_t)first, range[2 * i + 1] = (uint32_t)last;
   int dep = dnode >= bits ? L : dnode / ndim;
-  depth[i] = (uint8_t)(dep > L ? L : dep);
+  dep = dep > L ? L : dep;
+  depth[i] = (uint8_t)dep;
+  return make_uint3((uint32_t)first, (uint32_t)last, (uint32_t)dep);
 }
 
 // The binary radix tree over the sorted keys (karras_node): thread i takes internal node i, gathers
@@ -514,7 +571,7 @@ __global__ void __launch_bounds__(kThreads) k_build(
     block_prefix4(wrec, wsum, wtot, i < n ? i : -1);
   if (PART == 1 || i >= n - 1) return;
   omask[i] = 0u;  // k_frontier marks the octants
-  karras_node(k, lo, hi, ki, up, dn, i, ndim, left, right, parent, leaf_parent, range, depth);
+  karras_node<false>(k, lo, hi, ki, up, dn, i, ndim, left, right, parent, leaf_parent, range, depth);
 }
 
 // Every binary node below the root that is a d3 child (a point, or an internal node deeper than
@@ -522,16 +579,14 @@ __global__ void __launch_bounds__(kThreads) k_build(
 // binary nodes of equal depth, and marks its octant (its keys' digit at the parent's depth) in
 // the head's octant mask. Returns head | octant << 27 | 1 << 31 for the slots, 0 for other nodes.
 // pt: x is a point (sorted order), else an internal node.
-__device__ __forceinline__ uint32_t frontier_of(bool pt, uint32_t x, int ndim, const uint64_t* skeys,
-                                                const uint32_t* parent, const uint32_t* leaf_parent,
-                                                const uint32_t* range, const uint8_t* depth,
-                                                uint32_t* omask, uint32_t* err) {
+// p: its binary parent; first_of(): its first point.
+template <class First>
+__device__ __forceinline__ uint32_t frontier_of(bool pt, uint32_t x, uint32_t p, First first_of, int ndim,
+                                                const uint64_t* skeys, const uint32_t* parent,
+                                                const uint8_t* depth, uint32_t* omask, uint32_t* err) {
   // the parent cell's binary node: none for a graph's root, an index between two graphs, or a
   // point alone in its graph
-  uint32_t p = kNoParent;
-  if (pt) p = leaf_parent[x];
-  else if (depth[x] != kGapDepth && parent[x] != x) p = parent[x];
-  if (p == kNoParent) return 0u;
+  if (p == kNoParent || (!pt && (p == x || depth[x] == kGapDepth))) return 0u;
   const int Dp = depth[p];
   if (!pt && depth[x] <= Dp) return 0u;
   uint32_t h = p;
@@ -546,7 +601,7 @@ __device__ __forceinline__ uint32_t frontier_of(bool pt, uint32_t x, int ndim, c
   }
   uint32_t oct = 0;
   if (Dp < levels_of(ndim)) {
-    const uint64_t k = skeys[pt ? x : range[2 * x]];
+    const uint64_t k = skeys[first_of()];
     oct = (uint32_t)(k >> (64 - ndim * (Dp + 1))) & ((1u << ndim) - 1u);
     atomicOr(omask + h, (1u << oct) | (pt ? 0u : 1u << (16 + oct)));  // cells also above
   }
@@ -562,8 +617,9 @@ __global__ void __launch_bounds__(kThreads) k_frontier(
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 2 * n - 1) return;
   const bool pt = t >= n - 1;
-  head_of[t] = frontier_of(pt, pt ? (uint32_t)(t - (n - 1)) : (uint32_t)t, ndim, skeys, parent, leaf_parent,
-                           range, depth, omask, err);
+  const uint32_t x = pt ? (uint32_t)(t - (n - 1)) : (uint32_t)t;
+  head_of[t] = frontier_of(pt, x, pt ? leaf_parent[x] : parent[x], [&] { return pt ? x : range[2 * x]; }, ndim,
+                           skeys, parent, depth, omask, err);
 }
 
 // Exclusive prefix of the block totals, in place, by one block of kTopThreads: each thread sums
@@ -629,28 +685,16 @@ __device__ __forceinline__ uint32_t first_slot(const uint32_t* first, const uint
   return roots + first[x] + ctot[x >> 8];
 }
 
-// The cell of head i from the prefix sums (strengths of one sign, `sign`): its centroid and its
-// value at its own depth, in closed form.
-__device__ __forceinline__ float4 closed_cell(uint32_t i, int ndim, float sign,
-                                              const uint32_t* __restrict__ range,
-                                              const uint8_t* __restrict__ depth,
-                                              const D4* __restrict__ P, const D4* __restrict__ Ptot,
-                                              const float4* __restrict__ leaf,
-                                              const float* __restrict__ cube1, int fx_exp,
-                                              const FlSegs& seg) {
-  const uint32_t a = range[2 * i], b = range[2 * i + 1];
-  const float* cube = seg.graphs ? seg.g[seg.gid_pos[a]].origin : cube1;
-  const int fe = seg.graphs ? seg.g[seg.gid_pos[a]].fx : fx_exp;
-  // prefix sums: within the 256-point block, plus the blocks before it; exact in fixed point
-  const D4 hi = add4(P[b], Ptot[b >> 8]);
-  const D4 lo = a ? add4(P[a - 1], Ptot[(a - 1) >> 8]) : mk4(0, 0, 0, 0);
+// The cell of a head of depth D in closed form (strengths of one sign, `sign`): its centroid and its
+// value at its own depth. hi, lo: the prefix sums up to its last point and before its first, p0; in
+// fixed point, exact.
+__device__ __forceinline__ float4 closed_cell(D4 hi, D4 lo, float4 p0, int D, int ndim, float sign,
+                                              const float* __restrict__ cube, int fe) {
   const long long W = wsub(hi.x, lo.x);
-  const int D = depth[i];
   float4 out;
   if (W > 0) {
     // centroid = p0 + size * sum(w (u - u0)) / sum(w), about the range's first point p0: the
     // integer sums give the offsets exactly, so FP32 keeps the precision of the cell, not the cube
-    const float4 p0 = leaf[a];
     const float fW = ll2f_rn(W);
     const float sF = offset_scale(cube), r = cube[3] / fW;
     out.x = p0.x + ll2f_rn(wsub(wsub(hi.y, lo.y), mulhi62(W, fx_offset(p0.x, cube[0], sF)))) * r;
@@ -658,25 +702,24 @@ __device__ __forceinline__ float4 closed_cell(uint32_t i, int ndim, float sign,
     out.z = ndim > 2 ? p0.z + ll2f_rn(wsub(wsub(hi.w, lo.w), mulhi62(W, fx_offset(p0.z, cube[2], sF)))) * r : 0.f;
     out.w = sign * fW * __int_as_float((127 - fe) << 23) * damp(ndim, -D);
   } else {
-    out = leaf[a];
+    out = p0;
     out.w = 0.f;
   }
   return out;
 }
 
-// The d3 children of the cell that internal node i heads (its occupied octants; at the deepest level,
-// where the keys are equal, its points); 0 when i heads none.
-__device__ __forceinline__ uint32_t head_children(uint32_t i, int ndim, const uint32_t* parent,
-                                                  const uint32_t* range, const uint8_t* depth,
-                                                  const uint32_t* omask) {
-  const int D = depth[i];
-  if (D == kGapDepth) return 0u;
-  const uint32_t pa = parent[i];
-  if (!(pa == i || depth[pa] < D)) return 0u;  // a graph's root, or a deeper cell
-  return D >= levels_of(ndim) ? range[2 * i + 1] - range[2 * i] + 1 : (uint32_t)__popc(omask[i] & 0xffffu);
+// Whether internal node i of depth D, binary parent pa, heads a d3 cell: a graph's root, or the first
+// node of a deeper cell.
+__device__ __forceinline__ bool is_head(uint32_t i, int D, uint32_t pa, const uint8_t* depth) {
+  return D != kGapDepth && (pa == i || depth[pa] < D);
+}
+// The d3 children of a head's cell: its occupied octants; at the deepest level, where the keys are
+// equal, its points.
+__device__ __forceinline__ uint32_t children_of(int D, int ndim, uint32_t om, uint32_t points) {
+  return D >= levels_of(ndim) ? points : (uint32_t)__popc(om & 0xffffu);
 }
 
-// Every head's count of children (head_children); the counts' exclusive prefix within the block (first[]) and the block's total (ctot[]), for the slots. CLOSED (strengths
+// Every head's count of children; the counts' exclusive prefix within the block (first[]) and the block's total (ctot[]), for the slots. CLOSED (strengths
 // of one sign): a head's cell from the prefix sums too (closed_cell), into cell[].
 template <bool CLOSED>
 __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
@@ -698,11 +741,19 @@ __global__ void __launch_bounds__(kThreads) k_heads(int n, int ndim,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t c = 0;
   if (i < n - 1) {
-    c = head_children((uint32_t)i, ndim, parent, range, depth, omask);
-    if (!CLOSED) arrive[i] = 0u;  // the recursion's arrivals
+    const int D = depth[i];
+    if (is_head((uint32_t)i, D, parent[i], depth)) {
+      const uint32_t a = range[2 * i], b = range[2 * i + 1];
+      c = children_of(D, ndim, omask[i], b - a + 1);
+      if (CLOSED && c) {
+        const FlGraph* gr = seg.graphs ? seg.g + seg.gid_pos[a] : nullptr;
+        // prefix sums: within the 256-point block, plus the blocks before it
+        cell[i] = closed_cell(add4(P[b], Ptot[b >> 8]), a ? add4(P[a - 1], Ptot[(a - 1) >> 8]) : mk4(0, 0, 0, 0),
+                              leaf[a], D, ndim, sign, gr ? gr->origin : cube, gr ? gr->fx : fx_exp);
+      }
+    }
     count[i] = c;
-    if (CLOSED && c)
-      cell[i] = closed_cell((uint32_t)i, ndim, sign, range, depth, P, Ptot, leaf, cube, fx_exp, seg);
+    if (!CLOSED) arrive[i] = 0u;  // the recursion's arrivals
   }
   uint32_t x = c;
 #pragma unroll
@@ -998,7 +1049,7 @@ struct SmallTree {
 };
 
 // the keys among sorted a[0, len) before key: the smaller ones, and the equal ones with ties
-__device__ __forceinline__ uint32_t keys_before(const uint64_t* a, int len, uint64_t key, bool ties, int top) {
+__device__ __forceinline__ int keys_before(const uint64_t* a, int len, uint64_t key, bool ties, int top) {
   int at = 0;
   for (int step = top; step; step >>= 1) {
     const int q = at + step;
@@ -1007,12 +1058,22 @@ __device__ __forceinline__ uint32_t keys_before(const uint64_t* a, int len, uint
       if (o < key || (ties && o == key)) at = q;
     }
   }
-  return (uint32_t)at;
+  return at;
+}
+
+__host__ __device__ constexpr int small_align(int n) { return (n + 15) & ~15; }  // entries, to whole vectors
+// bytes of global memory into shared memory by a whole block, 16 at a time (the arrays' ends are padded)
+__device__ __forceinline__ void to_shared(void* dst, const void* src, int bytes) {
+  for (int j = threadIdx.x; j * 16 < bytes; j += blockDim.x)
+    reinterpret_cast<uint4*>(dst)[j] = reinterpret_cast<const uint4*>(src)[j];
 }
 
 template <bool CLOSED>
 __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree a) {
-  extern __shared__ uint64_t s_key[];  // [max(n, 1.5 slice)]: a slice's pairs in exchange, then all keys
+  // a slice's pairs in exchange; then every sorted key, and every node's parent and depth
+  extern __shared__ __align__(16) uint64_t s_key[];
+  uint32_t* s_parent = reinterpret_cast<uint32_t*>(s_key + small_align(a.t.n));
+  uint8_t* s_depth = reinterpret_cast<uint8_t*>(s_parent + small_align(a.t.n));
   __shared__ float s_cube[5];
   __shared__ D4 s_warp4[kSmallMaxThreads / 32];
   __shared__ uint32_t s_warp[kSmallMaxThreads / 32];
@@ -1030,9 +1091,9 @@ __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree
   };
   const uint32_t idx0 = (uint32_t)i;
   float4 p = ok ? a.pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  if (tid == 0) {
+  if (warp == 0) {
     d3_cover(a.red, ndim, s_cube);
-    if (c == 0)
+    if (c == 0 && lane == 0)
       for (int k = 0; k < 5; ++k) a.cube[k] = s_cube[k];
   }
   if (a.zero && c == C - 1)
@@ -1062,7 +1123,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree
     __syncthreads();
     s_key[tid] = key;
     __syncthreads();
-    uint32_t at = (uint32_t)r;
+    int at = r;
     for (int q = 0; q < S; q += kSmallRun)
       if (q != tid - r) at += keys_before(s_key + q, kSmallRun, key, q < tid - r, kSmallRun);
     __syncthreads();
@@ -1070,25 +1131,27 @@ __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree
     __syncthreads();
     key = s_key[tid], idx = s_idx[tid];
   }
+  if (ok) {
+    p = a.pos[idx];
+    p.w = a.strength[idx];
+  }
   if (C > 1) {
     if (ok) a.tmp[i] = key;
     sync();
-    for (int j = tid; j < n; j += S) s_key[j] = a.tmp[j];
+    to_shared(s_key, a.tmp, 8 * n);
     __syncthreads();
   }
   if (ok) {
-    uint32_t at = (uint32_t)tid;
+    int place = tid;
     for (int q = 0; q < used; ++q)
-      if (q != c)
-        at += keys_before(s_key + q * S, min(S, n - q * S), key, q < c, S >= 512 ? 512 : 256);
-    a.keys[at] = key;
-    a.perm[at] = idx;
-    p = a.pos[idx];
-    p.w = a.strength[idx];
-    a.t.leaf[at] = p;
+      if (q != c) place += keys_before(s_key + q * S, min(S, n - q * S), key, q < c, S >= 512 ? 512 : 256);
+    a.keys[place] = key;
+    a.perm[place] = idx;
+    a.t.leaf[place] = p;
   }
   sync();
-  for (int j = tid; j < n; j += S) s_key[j] = a.keys[j];
+  if (ok) p = a.t.leaf[i];
+  to_shared(s_key, a.keys, 8 * n);
   __syncthreads();
   // ---- the binary tree, and the points' records
   key = ok ? s_key[i] : 0;
@@ -1096,7 +1159,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree
   const int dn = ok ? kdelta(s_key, 0, n - 1, key, i, i - 1) : -1;
   if (CLOSED) {
     D4 v = mk4(0, 0, 0, 0);
-    if (ok) v = point_record(a.t.leaf[i], up, dn, ndim, s_cube, a.fx_exp);
+    if (ok) v = point_record(p, up, dn, ndim, s_cube, a.fx_exp);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const D4 y = shfl_up4(v, o);
@@ -1108,35 +1171,49 @@ __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree
     if (ok) reinterpret_cast<D4*>(a.t.wsum)[i] = v;
     if (tid == S - 1 && c < used) reinterpret_cast<D4*>(a.t.wtiles)[c] = v;
   }
+  uint3 me = make_uint3(0u, 0u, (uint32_t)kGapDepth);  // the node's first and last point, its depth
   if (node) {
     a.t.omask[i] = 0u;
     if (!CLOSED) a.t.flag[i] = 0u;
-    karras_node(s_key, 0, n - 1, key, up, dn, i, ndim, a.t.left, a.t.right, a.t.parent, a.t.leaf_parent,
-                a.t.range, a.t.depth);
+    if (S == kSmallRun)
+      me = karras_node<true>(s_key, 0, n - 1, key, up, dn, i, ndim, a.t.left, a.t.right, a.t.parent,
+                             a.t.leaf_parent, a.t.range, a.t.depth);
+    else
+      me = karras_node<false>(s_key, 0, n - 1, key, up, dn, i, ndim, a.t.left, a.t.right, a.t.parent,
+                              a.t.leaf_parent, a.t.range, a.t.depth);
   }
   sync();
-  // ---- the heads of the children's cells
-  const uint32_t nrec = node ? frontier_of(false, i, ndim, s_key, a.t.parent, a.t.leaf_parent, a.t.range,
-                                           a.t.depth, a.t.omask, a.err) : 0u;
-  const uint32_t prec = ok ? frontier_of(true, i, ndim, s_key, a.t.parent, a.t.leaf_parent, a.t.range,
-                                         a.t.depth, a.t.omask, a.err) : 0u;
-  if (!CLOSED && node) a.t.head_of[i] = nrec;
+  // ---- the heads of the children's cells, and the heads' cells
+  const uint32_t up_point = ok ? a.t.leaf_parent[i] : kNoParent;
+  const D4* P = reinterpret_cast<const D4*>(a.t.wsum);
+  D4 hi = mk4(0, 0, 0, 0), lo = mk4(0, 0, 0, 0);
+  float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (CLOSED && node) {  // for its cell, if it heads one: loads on their way beside the copies
+    hi = P[me.y], p0 = a.t.leaf[me.x];
+    if (me.x) lo = P[me.x - 1];
+  }
+  to_shared(s_parent, a.t.parent, 4 * (n - 1));
+  to_shared(s_depth, a.t.depth, n - 1);
   if (CLOSED && tid < (n + 255) / 256) {  // the records of the blocks before, per 256 points
     D4 b = mk4(0, 0, 0, 0);
     for (int q = 0; q < tid * 256 / S; ++q) b = add4(b, reinterpret_cast<const D4*>(a.t.wtiles)[q]);
     s_base4[tid] = b;
   }
-  sync();
-  // ---- the heads' children counted, their cells, and their first slots
-  uint32_t cnt = 0;
+  __syncthreads();
+  const uint32_t nrec = node ? frontier_of(false, i, s_parent[i], [&] { return me.x; }, ndim, s_key, s_parent,
+                                           s_depth, a.t.omask, a.err) : 0u;
+  const uint32_t prec = ok ? frontier_of(true, i, up_point, [&] { return (uint32_t)i; }, ndim, s_key, s_parent,
+                                         s_depth, a.t.omask, a.err) : 0u;
+  if (!CLOSED && node) a.t.head_of[i] = nrec;
+  const bool head = node && is_head((uint32_t)i, (int)me.z, s_parent[i], s_depth);
   float4 cell = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (node) {
-    cnt = head_children((uint32_t)i, ndim, a.t.parent, a.t.range, a.t.depth, a.t.omask);
-    a.t.count[i] = cnt;
-    if (CLOSED && cnt)
-      cell = closed_cell((uint32_t)i, ndim, a.sign, a.t.range, a.t.depth,
-                         reinterpret_cast<const D4*>(a.t.wsum), s_base4, a.t.leaf, s_cube, a.fx_exp, FlSegs{});
-  }
+  if (CLOSED && head)
+    cell = closed_cell(add4(hi, s_base4[me.y >> 8]), me.x ? add4(lo, s_base4[(me.x - 1) >> 8]) : lo, p0,
+                       (int)me.z, ndim, a.sign, s_cube, a.fx_exp);
+  sync();
+  // ---- the heads' children counted, and their first slots
+  const uint32_t cnt = head ? children_of((int)me.z, ndim, a.t.omask[i], me.y - me.x + 1) : 0u;
+  if (node) a.t.count[i] = cnt;
   uint32_t x = cnt;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -1160,15 +1237,14 @@ __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree
   double* slot64 = a.slots64 ? a.t.slot64 : nullptr;
   if (i == 0) {  // the root's own slot
     if (CLOSED) a.t.child_data[0] = cell;
-    a.t.child_meta[0] = make_uint2(first_slot(a.t.first, s_base, 0u, 1u), cnt | ((uint32_t)a.t.depth[0] << 26));
+    a.t.child_meta[0] = make_uint2(first_slot(a.t.first, s_base, 0u, 1u), cnt | (me.z << 26));
   }
   if (node)
-    write_slot<CLOSED>(false, i, nrec, n, ndim, 1u, a.t.omask, a.t.range, a.t.depth, a.t.count, a.t.first,
+    write_slot<CLOSED>(false, i, nrec, n, ndim, 1u, a.t.omask, a.t.range, s_depth, a.t.count, a.t.first,
                        s_base, &cell, a.t.child_data, a.t.child_meta, slot64, a.err);
   if (ok) {
-    const float4 l = a.t.leaf[i];
-    write_slot<CLOSED>(true, i, prec, n, ndim, 1u, a.t.omask, a.t.range, a.t.depth, a.t.count, a.t.first,
-                       s_base, &l, a.t.child_data, a.t.child_meta, slot64, a.err);
+    write_slot<CLOSED>(true, i, prec, n, ndim, 1u, a.t.omask, a.t.range, s_depth, a.t.count, a.t.first,
+                       s_base, &p, a.t.child_data, a.t.child_meta, slot64, a.err);
   }
 }
 
@@ -2104,8 +2180,8 @@ void fl_launch_small_tree(const FlTreeBufs* t, const FlSortBufs* sb, const float
   a.slots64 = !closed && fp64_depth != 0;
   static std::atomic<uint64_t> configured{0};
   if (fl_first_on_device(configured)) {
-    cudaFuncSetAttribute(k_small_tree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kSmallTreeMax);
-    cudaFuncSetAttribute(k_small_tree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kSmallTreeMax);
+    cudaFuncSetAttribute(k_small_tree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 13 * kSmallTreeMax);
+    cudaFuncSetAttribute(k_small_tree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 13 * kSmallTreeMax);
   }
   const int slice = kSmallRun * ((n + kSmallRun * kSmallBlocks - 1) / (kSmallRun * kSmallBlocks));
   int blocks = 1;
@@ -2113,7 +2189,7 @@ void fl_launch_small_tree(const FlTreeBufs* t, const FlSortBufs* sb, const float
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)slice);
-  cfg.dynamicSmemBytes = (size_t)(8 * n > 12 * slice ? 8 * n : 12 * slice);
+  cfg.dynamicSmemBytes = (size_t)(13 * small_align(n) > 12 * slice ? 13 * small_align(n) : 12 * slice);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2317,9 +2393,7 @@ void fl_launch_allpairs(const float4* pos, const float* strength, float4* vel, i
 
 void fl_launch_bgraph(int graphs, int ndim, const int32_t* off, const FlReduce* red,
                       const FlBatchParams* prm, const double* alpha, FlGraph* gr, cudaStream_t st) {
-  // one warp a block: the covers are FP64, a warp instruction of which holds its SM's pipe for 16
-  // clocks, so the warps want an SM each (256 graphs in one block took 14 us)
-  k_bgraph<<<(graphs + 31) / 32, 32, 0, st>>>(graphs, ndim, off, red, prm, alpha, gr);
+  k_bgraph<<<(graphs + 3) / 4, 128, 0, st>>>(graphs, ndim, off, red, prm, alpha, gr);
 }
 
 void fl_launch_bmorton(const float4* pos, int n, int ndim, const uint32_t* gid, const FlGraph* gr,
