@@ -79,6 +79,8 @@ void fl_launch_bgather(int n, const uint32_t* order2, const uint64_t* mkeys, con
 struct FlSortBufs {
   uint64_t* keys[2];
   uint32_t* vals[2];
+  const uint64_t* in_keys;  // where the first pass and the histogram read, if not keys[0] / vals[0]
+  const uint32_t* in_vals;
   uint32_t* hist;      // [8][256] digit counts per pass
   uint32_t* status;    // [passes][tiles][256] look-back words (tiles of this sort's tile size)
   uint32_t* counters;  // [kSortCounters]: tile tickets of up to 8 passes, then the run fix-up's

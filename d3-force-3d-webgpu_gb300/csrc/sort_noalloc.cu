@@ -30,13 +30,15 @@ constexpr int64_t kMaxPairs = FL_SORT_NOALLOC_MAX_PAIRS;
 constexpr int64_t kTiles = kSortTilesSmall;  // the most tiles of a sort of up to kMaxPairs pairs
 static_assert(kMaxPairs <= kTiles * kSortTileMid, "more pairs have more tiles");
 constexpr size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
-constexpr size_t kErrOff = 0;
-constexpr size_t kKeysOff = 256;
+// the error word, the histograms, the tickets and the look-back words in that order: one memset
+// clears what a sort uses
+constexpr size_t kKeysOff = 0;
 constexpr size_t kValsOff = kKeysOff + a256(8 * (size_t)kMaxPairs);
-constexpr size_t kHistOff = kValsOff + a256(4 * (size_t)kMaxPairs);
-constexpr size_t kStatusOff = kHistOff + a256(8 * 256 * 4);
-constexpr size_t kCountersOff = kStatusOff + a256(8 * (size_t)kTiles * 256 * 4);
-constexpr size_t kScratchBytes = kCountersOff + 256;  // 3.6 MB for 262,144 pairs
+constexpr size_t kErrOff = kValsOff + a256(4 * (size_t)kMaxPairs);
+constexpr size_t kHistOff = kErrOff + 256;
+constexpr size_t kCountersOff = kHistOff + a256(8 * 256 * 4);
+constexpr size_t kStatusOff = kCountersOff + 256;
+constexpr size_t kScratchBytes = kStatusOff + a256(8 * (size_t)kTiles * 256 * 4);  // 4.2 MB for 262,144 pairs
 
 static __device__ __align__(256) unsigned char g_sort_scratch[kScratchBytes];
 
@@ -91,10 +93,16 @@ extern "C" int32_t fl_radix_sort_noalloc(const uint64_t* keys, const uint32_t* v
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   uint32_t* err = reinterpret_cast<uint32_t*>(base + kErrOff);
   FlSortBufs sb{};
-  sb.keys[0] = keys_out;
-  sb.vals[0] = vals_out;
-  sb.keys[1] = reinterpret_cast<uint64_t*>(base + kKeysOff);
-  sb.vals[1] = reinterpret_cast<uint32_t*>(base + kValsOff);
+  // Buffers apart: the first pass reads the caller's input, and writes the half from which the last
+  // one ends in the output. A sort in place starts in the output.
+  const int passes = (64 - lo_bit + 7) / 8;
+  const bool apart = keys != keys_out && vals != vals_out;
+  const int out = apart ? passes & 1 : 0;
+  if (apart) sb.in_keys = keys, sb.in_vals = vals;
+  sb.keys[out] = keys_out;
+  sb.vals[out] = vals_out;
+  sb.keys[1 - out] = reinterpret_cast<uint64_t*>(base + kKeysOff);
+  sb.vals[1 - out] = reinterpret_cast<uint32_t*>(base + kValsOff);
   sb.hist = reinterpret_cast<uint32_t*>(base + kHistOff);
   sb.status = reinterpret_cast<uint32_t*>(base + kStatusOff);
   sb.counters = reinterpret_cast<uint32_t*>(base + kCountersOff);
@@ -106,19 +114,19 @@ extern "C" int32_t fl_radix_sort_noalloc(const uint64_t* keys, const uint32_t* v
   cudaError_t e;
   // every call shares the scratch and finds the last call's contents: the error word, the
   // histograms, the look-back words and the tickets must start at zero
-  if ((e = cudaMemsetAsync(err, 0, 4, st)) != cudaSuccess ||
-      (e = cudaMemsetAsync(base + kHistOff, 0, kScratchBytes - kHistOff, st)) != cudaSuccess)
-    return cuda_fail(e, "cudaMemsetAsync");
-  if (keys != keys_out && (e = cudaMemcpyAsync(keys_out, keys, kb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+  const int64_t tiles = (n + fl_sort_tile(n) - 1) / fl_sort_tile(n);
+  const size_t used = kStatusOff + (size_t)passes * tiles * 256 * 4 - kErrOff;
+  if ((e = cudaMemsetAsync(err, 0, used, st)) != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
+  if (!apart && keys != keys_out && (e = cudaMemcpyAsync(keys_out, keys, kb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
     return cuda_fail(e, "cudaMemcpyAsync");
-  if (vals != vals_out && (e = cudaMemcpyAsync(vals_out, vals, vb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+  if (!apart && vals != vals_out && (e = cudaMemcpyAsync(vals_out, vals, vb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
     return cuda_fail(e, "cudaMemcpyAsync");
   fl_sort_histogram(&sb, n, lo_bit, st, &launches);
   const int r = fl_sort_passes(&sb, n, lo_bit, err, st, &launches);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "sort launch");
-  if (r == 1) {  // an odd number of digit passes ends in the scratch half
-    if ((e = cudaMemcpyAsync(keys_out, sb.keys[1], kb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(vals_out, sb.vals[1], vb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
+  if (r != out) {  // in place, an odd number of digit passes ends in the scratch half
+    if ((e = cudaMemcpyAsync(keys_out, sb.keys[1 - out], kb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(vals_out, sb.vals[1 - out], vb, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
       return cuda_fail(e, "cudaMemcpyAsync");
   }
   uint32_t w = 0;
