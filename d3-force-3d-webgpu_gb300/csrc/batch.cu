@@ -169,10 +169,12 @@ void encode_batch_tick(fl_batch* b, const double* alpha, const FlTick* tk) {
                       b->sb.hist, lo_sort, ts);
     int r = fl_sort_passes(&b->sb, n, lo_sort, err, ts, &b->launches);
     r = fl_sort_runfix(&b->sb, n, lo_bit, lo_sort, r, ts, &b->launches);
-    fl_sort_reset(&b->sb2, n, 2, ts);
-    fl_launch_bgidkey(n, b->sb.vals[r], gid, b->off.as<int32_t>(), G, b->sb2.keys[0],
+    // digit passes over the graphs: one for up to 256 of them (a pass over 1M points takes 15 us)
+    const int gid_passes = G > 256 ? 2 : 1;
+    fl_sort_reset(&b->sb2, n, gid_passes, ts);
+    fl_launch_bgidkey(n, b->sb.vals[r], gid, b->off.as<int32_t>(), G, gid_passes, b->sb2.keys[0],
                       b->sb2.vals[0], b->sb2.hist, ts);
-    const int r2 = fl_sort_passes(&b->sb2, n, 48, err, ts, &b->launches);
+    const int r2 = fl_sort_passes(&b->sb2, n, 64 - 8 * gid_passes, err, ts, &b->launches);
     skeys = b->sb.keys[1 - r];
     perm = b->sb.vals[1 - r];
     fl_launch_bgather(n, b->sb2.vals[r2], b->sb.keys[r], b->sb.vals[r], gid, skeys, perm, gpos, ts);

@@ -320,8 +320,8 @@ __global__ void __launch_bounds__(kMortonThreads) k_bmorton(const float4* __rest
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
-// The second sort's input: the graph of each point in Morton order, in key bits [48, 64), and
-// the point's Morton-order position; with the histograms of those two digits.
+// The second sort's input: the graph of each point in Morton order, in the top `passes` bytes of the
+// key, and the point's Morton-order position; with the histograms of those digits.
 // The graph of node `node`: the last g with off[g] <= node (graph offsets in shared memory).
 __device__ __forceinline__ uint32_t graph_of(const int32_t* s_off, int graphs, uint32_t node) {
   int lo = 0, hi = graphs - 1;
@@ -337,7 +337,7 @@ constexpr int kGidSearchMax = 8192;  // graphs whose offsets the key kernel sear
 __global__ void __launch_bounds__(kMortonThreads) k_bgidkey(int n, const uint32_t* __restrict__ mperm,
                                                       const uint32_t* __restrict__ gid,
                                                       const int32_t* __restrict__ off, int graphs,
-                                                      uint64_t* __restrict__ keys,
+                                                      int passes, uint64_t* __restrict__ keys,
                                                       uint32_t* __restrict__ vals,
                                                       uint32_t* __restrict__ hist) {
   __shared__ uint32_t sh[2 * 256];
@@ -355,12 +355,12 @@ __global__ void __launch_bounds__(kMortonThreads) k_bgidkey(int n, const uint32_
     if (ok) {
       // a node's graph: from the offsets (a search in shared memory) rather than a random read
       const uint32_t node = mperm[i];
-      key = (uint64_t)(search ? graph_of(s_off, graphs, node) : gid[node]) << 48;
+      key = (uint64_t)(search ? graph_of(s_off, graphs, node) : gid[node]) << (64 - 8 * passes);
       keys[i] = key;
       vals[i] = (uint32_t)i;
     }
-    fl::hist_add(sh, (uint32_t)(key >> 48) & 255u, ok);
-    fl::hist_add(sh + 256, (uint32_t)(key >> 56) & 255u, ok);
+    for (int p = 0; p < passes; ++p)
+      fl::hist_add(sh + p * 256, (uint32_t)(key >> (64 - 8 * (passes - p))) & 255u, ok);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 2 * 256; i += blockDim.x)
@@ -2405,13 +2405,14 @@ void fl_launch_bmorton(const float4* pos, int n, int ndim, const uint32_t* gid, 
 }
 
 void fl_launch_bgidkey(int n, const uint32_t* mperm, const uint32_t* gid, const int32_t* off,
-                       int graphs, uint64_t* keys, uint32_t* vals, uint32_t* hist, cudaStream_t st) {
+                       int graphs, int passes, uint64_t* keys, uint32_t* vals, uint32_t* hist,
+                       cudaStream_t st) {
   // as fl_launch_morton: few, large blocks (each flushes its histograms with global atomics
   // and loads the graph offsets once)
   int g = (n + kMortonThreads - 1) / kMortonThreads;
   if (g > 2 * fl_sms()) g = 2 * fl_sms();
   if (g < 1) g = 1;
-  k_bgidkey<<<g, kMortonThreads, 0, st>>>(n, mperm, gid, off, graphs, keys, vals, hist);
+  k_bgidkey<<<g, kMortonThreads, 0, st>>>(n, mperm, gid, off, graphs, passes, keys, vals, hist);
 }
 
 void fl_launch_bgather(int n, const uint32_t* order2, const uint64_t* mkeys, const uint32_t* mperm,
