@@ -66,7 +66,7 @@ WALK_BYTES_PER_NODE = 16 + 4 + 48 + 32
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one walk launch of the default
 # 1M-node workload, from an ncu capture of that launch: a profiler figure, not something this
 # run can measure, so it is reported at that size only, with where it came from
-WALK_DRAM_BYTES_1M = 74.4e6
+WALK_DRAM_BYTES_1M = 74.8e6
 WALK_DRAM_SOURCE = "ncu --set full capture of one k_walk launch, 1M-node workload"
 FLOPS_PER_INTERACTION = 20  # FP32 ops per accepted cell or point interaction
 FLOPS_PER_OPEN = 8          # per opened-cell test

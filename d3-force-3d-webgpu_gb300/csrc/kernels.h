@@ -250,7 +250,7 @@ void fl_launch_aggregate(const FlTreeBufs* t, const uint64_t* skeys, bool closed
                          cudaStream_t st, int64_t* launches, FlSegs segs = FlSegs{});
 // Scale exponent of the fixed-point cell sums: no sum over n points of weight <= wmax overflows.
 int fl_fixed_exponent(int64_t n, double wmax);
-// stats (optional): [0] child tests made by the warps (32 per child), [1] of those, tests by a
+// stats (optional): [0] child tests made by the warps (one per child and point of the group), [1] of those, tests by a
 // lane whose point needed them (the d3 traversal's own work)
 // group: points per traversal (16 or 32), 1 for one point per warp with the lanes over the
 // point's children (small layouts), 0 for the default by size (fl_walk_group_for)

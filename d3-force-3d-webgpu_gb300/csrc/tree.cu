@@ -35,6 +35,8 @@
 //              w^2 / theta^2 < l, points are summed exactly, distanceMin / distanceMax as d3;
 //              cells that some point must open are pushed with the mask of those points.
 //
+// Up to 6,144 points, morton to slots are one launch (k_small_tree).
+//
 // Points with the same code at the finest level share the deepest cell as its children.
 #include <cooperative_groups.h>
 #include <math.h>

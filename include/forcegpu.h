@@ -321,7 +321,7 @@ int32_t fl_radix_sort(const uint64_t* keys, const uint32_t* vals, int64_t n, int
  * DEVICE buffers of n pairs on the calling thread's current device (the outputs may be the
  * inputs, sorted in place; they must not otherwise overlap); the sort runs on `stream` (NULL:
  * the default stream) and the call returns when it has finished. Its scratch is a built-in
- * device array of about 3.6 MB, present on every device that loads this library until the
+ * device array of about 4.2 MB, present on every device that loads this library until the
  * process exits, so n may not exceed FL_SORT_NOALLOC_MAX_PAIRS (FL_E_ARG otherwise). Every
  * call looks the array's address up in the current context (cudaGetSymbolAddress, which
  * allocates nothing); the first call in a context also loads the library's device code there:
