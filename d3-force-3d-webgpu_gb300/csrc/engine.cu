@@ -604,15 +604,23 @@ void encode_tick(fl_sim* s, float alpha, float decay) {
         ++s->launches;
         break;
       }
-      case FL_FORCE_POSITION:
-        if (p->d.axis < 0 || p->d.axis >= s->ndim) break;  // forceZ in 2D: nothing to act on
-        {
-          Scope sc(s, G_POSITION);
-          fl_launch_position(s->pos.as<float4>(), vel_cur(s), p->a.as<float>(), p->b.as<float>(),
-                             n, p->d.axis, alpha, s->st, s->tkp);
-          ++s->launches;
+      case FL_FORCE_POSITION: {
+        FlAxes f{};
+        for (; k < np && plan[k]->type == FL_FORCE_POSITION; ++k) {
+          const Pass* q = plan[k].get();
+          const int axis = q->d.axis;
+          if (axis < 0 || axis >= s->ndim) continue;  // forceZ in 2D: nothing to act on
+          if (f.axes >> axis & 1) break;  // an axis again: a launch of its own
+          f.axes |= 1 << axis;
+          f.target[axis] = q->a.as<float>(), f.strength[axis] = q->b.as<float>();
         }
+        --k;  // the last one taken
+        if (!f.axes) break;
+        Scope sc(s, G_POSITION);
+        fl_launch_position(s->pos.as<float4>(), vel_cur(s), f, n, alpha, s->st, s->tkp);
+        ++s->launches;
         break;
+      }
     }
   }
   {

@@ -153,8 +153,12 @@ void fl_launch_unpack(const float* src, int count, int ndim, float4* dst, cudaSt
 void fl_launch_radial(const float4* pos, float4* vel, const float* radius, const float* strength,
                       int n, int ndim, float cx, float cy, float cz, float alpha, cudaStream_t st,
                       const FlTick* tk = nullptr);
-void fl_launch_position(const float4* pos, float4* vel, const float* target, const float* strength,
-                        int n, int axis, float alpha, cudaStream_t st, const FlTick* tk = nullptr);
+struct FlAxes {  // position forces of different axes: bit a of axes, its targets and strengths
+  int axes;
+  const float *target[3], *strength[3];
+};
+void fl_launch_position(const float4* pos, float4* vel, const FlAxes& f, int n, float alpha, cudaStream_t st,
+                        const FlTick* tk = nullptr);
 
 // ---------------------------------------------------------------- link (link.cu)
 struct FlLinkCsr {
