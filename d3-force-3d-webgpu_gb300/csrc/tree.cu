@@ -1859,7 +1859,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
 // memory as pairs for the f32x2 arithmetic. Four sources at a time, for every point of the lane,
 // are tested for what is not the common case (the point itself, distanceMin, a zero component)
 // by the least of their squared distances and components, with one vote; such a four is summed
-// again source by source. The warps' sums are added in a fixed order, in shared memory and then
+// source by source. The common path weighs a source that does not count with 0, so its displacement
+// has to be finite: a source without strength is laid out at a place that no point meets, a tile with a
+// source beyond kPairFar (infinite or NaN too) is summed source by source, and a point beyond it is
+// given infinite coordinates, so that every source is infinitely far and tested apart. The warps' sums are added in a fixed order, in shared memory and then
 // over the cluster's.
 //
 // Bound by the FP32 pipe and instruction issue: a pair of sources takes 10 packed instructions of
@@ -1871,9 +1874,16 @@ constexpr int kPairThreads = 128;
 constexpr int kPairWarps = kPairThreads / 32;
 constexpr int kPairClusterMax = 8;
 constexpr int kPairTwoPoints = 10000;  // more points than this: two per lane
+constexpr float kPairFar = 8.5070592e37f;  // 2^126: no difference of coordinates below it overflows
+constexpr float kPairNowhere = 1.1529215e18f;  // 2^60: finite squares, and no subnormal distance nearby
+// whether a coordinate of p is kPairFar or more, infinite or NaN
+template <int NDIM>
+__device__ __forceinline__ bool pair_far(float4 p) {
+  return !(fabsf(p.x) < kPairFar) || (NDIM > 1 && !(fabsf(p.y) < kPairFar)) || (NDIM > 2 && !(fabsf(p.z) < kPairFar));
+}
 
 // One source's force on a point, every case.
-template <int NDIM, bool DMAX>
+template <int NDIM>
 __device__ __forceinline__ void pair_term(float4 me, uint32_t i, float4 o, uint32_t other,
                                           float dmin2, float dmax2, uint32_t step, uint32_t seed,
                                           float& ax, float& ay, float& az) {
@@ -1882,7 +1892,7 @@ __device__ __forceinline__ void pair_term(float4 me, uint32_t i, float4 o, uint3
   float l = dx * dx;
   if (NDIM > 1) l = fmaf(dy, dy, l);
   if (NDIM > 2) l = fmaf(dz, dz, l);
-  if (DMAX && l >= dmax2) return;
+  if (l >= dmax2) return;  // also without a distanceMax: an infinite distance
   if (dx == 0.f) dx = fl::jiggle(i, other, 0, step, seed), l += dx * dx;
   if (NDIM > 1 && dy == 0.f) dy = fl::jiggle(i, other, 1, step, seed), l += dy * dy;
   if (NDIM > 2 && dz == 0.f) dz = fl::jiggle(i, other, 2, step, seed), l += dz * dz;
@@ -1904,23 +1914,31 @@ __global__ void __launch_bounds__(kPairThreads) k_allpairs(
   const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first = (int)(blockIdx.x / blocks) * 32 * Q;
+  // l <= close: distanceMin, no distance at all, or (a far point) any
+  float close = fmaxf(below(dmin2), 0.f);
   float4 me[Q];
   uint64_t MX[Q], MY[Q], MZ[Q], AX[Q], AY[Q], AZ[Q];
 #pragma unroll
   for (int p = 0; p < Q; ++p) {
     const int i = first + 32 * p + lane;
     me[p] = i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    MX[p] = pk2(me[p].x, me[p].x), MY[p] = pk2(me[p].y, me[p].y), MZ[p] = pk2(me[p].z, me[p].z);
+    const bool far = pair_far<NDIM>(me[p]);
+    const float x = far ? INFINITY : me[p].x, y = far ? INFINITY : me[p].y, z = far ? INFINITY : me[p].z;
+    MX[p] = pk2(x, x), MY[p] = pk2(y, y), MZ[p] = pk2(z, z);
     AX[p] = AY[p] = AZ[p] = 0;
+    if (far) close = INFINITY;
   }
   constexpr int K = 2;  // pairs of sources at a time
-  const float close = fmaxf(below(dmin2), 0.f);  // l <= close: distanceMin, or no distance at all
   float4* sa = s_a[warp];
   float4* sb = s_b[warp];
   for (int base = 32 * (rank * kPairWarps + warp); base < n; base += 32 * kPairWarps * blocks) {
     const int j = base + lane;
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < n) o = pos[j], o.w = strength[j] * alpha;
+    float4 o = make_float4(kPairNowhere, kPairNowhere, kPairNowhere, 0.f);
+    if (j < n) {
+      const float w = strength[j];
+      if (w != 0.f) o = pos[j], o.w = w * alpha;
+    }
+    const bool one_by_one = __any_sync(FL_FULL, pair_far<NDIM>(o));
     __syncwarp();
     {
       float* pa = reinterpret_cast<float*>(&sa[lane >> 1]) + (lane & 1);
@@ -1953,11 +1971,11 @@ __global__ void __launch_bounds__(kPairThreads) k_allpairs(
           if (NDIM > 1) cmin = fminf(fminf(cmin, fabsf(dy.x)), fabsf(dy.y));
           if (NDIM > 2) cmin = fminf(fminf(cmin, fabsf(dz.x)), fabsf(dz.y));
         }
-      bool odd = lmin <= close || cmin == 0.f;
+      bool odd = one_by_one || lmin <= close || cmin == 0.f;
       // in a small layout mostly the point itself: then as if infinitely far (in a large one it is
       // met too seldom for what the test costs in registers)
       if (Q == 1 && __any_sync(FL_FULL, odd)) {
-        odd = false;
+        odd = one_by_one;
 #pragma unroll
         for (int c = 0; c < K; ++c) {
           const int self = first + lane - (base + 2 * (k + c));
@@ -1977,8 +1995,8 @@ __global__ void __launch_bounds__(kPairThreads) k_allpairs(
           for (int c = 0; c < K; ++c) {
             const float4 u = sa[k + c], v = sb[k + c];
             const uint32_t at = (uint32_t)(base + 2 * (k + c));
-            pair_term<NDIM, DMAX>(me[p], i, make_float4(u.x, u.z, v.x, v.z), at, dmin2, dmax2, step, seed, ax.x, ay.x, az.x);
-            pair_term<NDIM, DMAX>(me[p], i, make_float4(u.y, u.w, v.y, v.w), at + 1, dmin2, dmax2, step, seed, ax.y, ay.y, az.y);
+            pair_term<NDIM>(me[p], i, make_float4(u.x, u.z, v.x, v.z), at, dmin2, dmax2, step, seed, ax.x, ay.x, az.x);
+            pair_term<NDIM>(me[p], i, make_float4(u.y, u.w, v.y, v.w), at + 1, dmin2, dmax2, step, seed, ax.y, ay.y, az.y);
           }
           AX[p] = pk2(ax.x, ax.y), AY[p] = pk2(ay.x, ay.y), AZ[p] = pk2(az.x, az.y);
         }
