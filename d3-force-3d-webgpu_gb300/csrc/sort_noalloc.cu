@@ -63,6 +63,8 @@ int32_t scratch_of_current_context(char** out) {
   return FL_OK;
 }
 
+bool aligned(const void* p, uintptr_t to) { return reinterpret_cast<uintptr_t>(p) % to == 0; }
+
 bool overlap(const void* a, size_t an, const void* b, size_t bn) {
   const char *x = static_cast<const char*>(a), *y = static_cast<const char*>(b);
   return x < y + bn && y < x + an;
@@ -87,6 +89,8 @@ extern "C" int32_t fl_radix_sort_noalloc(const uint64_t* keys, const uint32_t* v
       (vals != vals_out && overlap(vals, vb, vals_out, vb)) || overlap(keys_out, kb, vals_out, vb) ||
       overlap(keys_out, kb, vals, vb) || overlap(vals_out, vb, keys, kb))
     return fail(FL_E_ARG, "input and output buffers overlap (only identical, in-place buffers may)");
+  if (!aligned(keys_out, 8) || !aligned(vals_out, 4))
+    return fail(FL_E_ARG, "the output buffers are not aligned to their elements");
   char* base = nullptr;
   int32_t rc = scratch_of_current_context(&base);
   if (rc) return rc;
@@ -94,9 +98,10 @@ extern "C" int32_t fl_radix_sort_noalloc(const uint64_t* keys, const uint32_t* v
   uint32_t* err = reinterpret_cast<uint32_t*>(base + kErrOff);
   FlSortBufs sb{};
   // Buffers apart: the first pass reads the caller's input, and writes the half from which the last
-  // one ends in the output. A sort in place starts in the output.
+  // one ends in the output. A sort in place starts in the output, and so does one of an input that is
+  // not aligned to its elements, which the kernels cannot read: it is copied there first.
   const int passes = (64 - lo_bit + 7) / 8;
-  const bool apart = keys != keys_out && vals != vals_out;
+  const bool apart = keys != keys_out && vals != vals_out && aligned(keys, 8) && aligned(vals, 4);
   const int out = apart ? passes & 1 : 0;
   if (apart) sb.in_keys = keys, sb.in_vals = vals;
   sb.keys[out] = keys_out;

@@ -319,8 +319,10 @@ int32_t fl_radix_sort(const uint64_t* keys, const uint32_t* vals, int64_t n, int
  * that must not stall the device with cudaMalloc/cudaFree, and those that must not fail for lack
  * of memory mid-frame. No counterpart in the reference. keys/vals and keys_out/vals_out are
  * DEVICE buffers of n pairs on the calling thread's current device (the outputs may be the
- * inputs, sorted in place; they must not otherwise overlap); the sort runs on `stream` (NULL:
- * the default stream) and the call returns when it has finished. Its scratch is a built-in
+ * inputs, sorted in place; they must not otherwise overlap). The outputs must be aligned to their
+ * elements (FL_E_ARG otherwise); an input apart from its output may start at any byte (one that is
+ * not aligned is copied first). The sort runs on `stream` (NULL: the default stream) and the call
+ * returns when it has finished. Its scratch is a built-in
  * device array of about 4.2 MB, present on every device that loads this library until the
  * process exits, so n may not exceed FL_SORT_NOALLOC_MAX_PAIRS (FL_E_ARG otherwise). Every
  * call looks the array's address up in the current context (cudaGetSymbolAddress, which
