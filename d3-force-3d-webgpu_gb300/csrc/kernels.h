@@ -120,9 +120,10 @@ int fl_sort_passes(const FlSortBufs* b, int64_t n, int lo_bit, uint32_t* err, cu
 int fl_sort_split(int lo_bit, int passes = 0);
 int fl_sort_runfix(const FlSortBufs* b, int64_t n, int lo_bit, int lo_sort, int cur,
                    cudaStream_t st, int64_t* launches);
-// True the first time it is called on the current device for `done` (a kernel's shared-memory
-// limit is raised once per device).
-bool fl_first_on_device(std::atomic<uint64_t>& done);
+// Raises a kernel's limit of dynamic shared memory on the current device, if `done` (the kernel's own)
+// does not say that it has been. A device is marked only after the call, so that a thread that finds the
+// mark can launch; threads that meet before it each make the call.
+void fl_raise_shared_limit(std::atomic<uint64_t>& done, const void* kernel, int bytes);
 
 // ---------------------------------------------------------------- state kernels (state.cu)
 void fl_launch_reduce(const float4* pos, int n, int ndim, int want_box, int want_sum,

@@ -397,8 +397,7 @@ void launch_pass(const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint3
                  uint32_t* err, uint32_t spin_limit, int hold, cudaStream_t st) {
   static std::atomic<uint64_t> configured{0};
   const size_t dyn = (size_t)T * I * 12;
-  if (fl_first_on_device(configured))
-    cudaFuncSetAttribute(k_onesweep<T, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  fl_raise_shared_limit(configured, (const void*)k_onesweep<T, I>, (int)dyn);
   const int64_t tiles = (n + T * I - 1) / (T * I);
   k_onesweep<T, I><<<(int)tiles, T, dyn, st>>>(kin, vin, kout, vout, n, shift, ghist, status,
                                                ticket, err, spin_limit, hold);
@@ -426,12 +425,14 @@ static FlSortShape sort_shape(int64_t n) {
   return {threads, it < 5 ? 5 : (int)it};
 }
 
-bool fl_first_on_device(std::atomic<uint64_t>& done) {
+void fl_raise_shared_limit(std::atomic<uint64_t>& done, const void* kernel, int bytes) {
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return true;
-  const uint64_t bit = 1ull << dev;
-  return !(done.fetch_or(bit) & bit);
+  const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return;
+  // a failure stays the thread's last error, which the caller reads after its launches
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+    done.fetch_or(bit, std::memory_order_release);
 }
 
 int fl_sort_tile(int64_t n) {

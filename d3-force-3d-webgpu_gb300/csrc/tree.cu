@@ -2201,11 +2201,10 @@ void fl_launch_small_tree(const FlTreeBufs* t, const FlSortBufs* sb, const float
   a.tmp = sb->keys[0], a.keys = sb->keys[1], a.vtmp = sb->vals[0], a.perm = sb->vals[1];
   a.cube = cube, a.err = err, a.t = *t, a.sign = sign, a.fx_exp = fx_exp;
   a.slots64 = !closed && fp64_depth != 0;
-  static std::atomic<uint64_t> configured{0};
-  if (fl_first_on_device(configured)) {
-    cudaFuncSetAttribute(k_small_tree<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 13 * kSmallTreeMax);
-    cudaFuncSetAttribute(k_small_tree<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 13 * kSmallTreeMax);
-  }
+  static std::atomic<uint64_t> configured[2];  // zero: static
+  // both kernels at the first launch, which is never inside a capture
+  fl_raise_shared_limit(configured[0], (const void*)k_small_tree<false>, 13 * kSmallTreeMax);
+  fl_raise_shared_limit(configured[1], (const void*)k_small_tree<true>, 13 * kSmallTreeMax);
   const int slice = kSmallRun * ((n + kSmallRun * kSmallBlocks - 1) / (kSmallRun * kSmallBlocks));
   int blocks = 1;
   while (blocks * slice < n) blocks *= 2;
