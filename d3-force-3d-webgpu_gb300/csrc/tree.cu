@@ -44,6 +44,7 @@
 #include <atomic>
 #include <cuda/atomic>
 #include <cmath>
+#include <type_traits>
 
 #include "kernels.h"
 
@@ -1860,9 +1861,9 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
 // are tested for what is not the common case (the point itself, distanceMin, a zero component)
 // by the least of their squared distances and components, with one vote; such a four is summed
 // source by source. The common path weighs a source that does not count with 0, so its displacement
-// has to be finite: a source without strength is laid out at a place that no point meets, a tile with a
-// source beyond kPairFar (infinite or NaN too) is summed source by source, and a point beyond it is
-// given infinite coordinates, so that every source is infinitely far and tested apart. The warps' sums are added in a fixed order, in shared memory and then
+// has to be finite: a source without strength is laid out at a place that no point meets, and a tile
+// with a source beyond kPairFar (infinite or NaN too), or for a point beyond it, is summed source by
+// source. The warps' sums are added in a fixed order, in shared memory and then
 // over the cluster's.
 //
 // Bound by the FP32 pipe and instruction issue: a pair of sources takes 10 packed instructions of
@@ -1882,8 +1883,9 @@ __device__ __forceinline__ bool pair_far(float4 p) {
   return !(fabsf(p.x) < kPairFar) || (NDIM > 1 && !(fabsf(p.y) < kPairFar)) || (NDIM > 2 && !(fabsf(p.z) < kPairFar));
 }
 
-// One source's force on a point, every case.
-template <int NDIM>
+// One source's force on a point, every case but, without DMAX, that of an infinite distance between
+// infinite coordinates, which is left out too (an infinite l of finite ones adds 0).
+template <int NDIM, bool DMAX>
 __device__ __forceinline__ void pair_term(float4 me, uint32_t i, float4 o, uint32_t other,
                                           float dmin2, float dmax2, uint32_t step, uint32_t seed,
                                           float& ax, float& ay, float& az) {
@@ -1892,7 +1894,7 @@ __device__ __forceinline__ void pair_term(float4 me, uint32_t i, float4 o, uint3
   float l = dx * dx;
   if (NDIM > 1) l = fmaf(dy, dy, l);
   if (NDIM > 2) l = fmaf(dz, dz, l);
-  if (l >= dmax2) return;  // also without a distanceMax: an infinite distance
+  if (DMAX && l >= dmax2) return;
   if (dx == 0.f) dx = fl::jiggle(i, other, 0, step, seed), l += dx * dx;
   if (NDIM > 1 && dy == 0.f) dy = fl::jiggle(i, other, 1, step, seed), l += dy * dy;
   if (NDIM > 2 && dz == 0.f) dz = fl::jiggle(i, other, 2, step, seed), l += dz * dz;
@@ -1914,31 +1916,29 @@ __global__ void __launch_bounds__(kPairThreads) k_allpairs(
   const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first = (int)(blockIdx.x / blocks) * 32 * Q;
-  // l <= close: distanceMin, no distance at all, or (a far point) any
-  float close = fmaxf(below(dmin2), 0.f);
+  bool far_point = false;
   float4 me[Q];
   uint64_t MX[Q], MY[Q], MZ[Q], AX[Q], AY[Q], AZ[Q];
 #pragma unroll
   for (int p = 0; p < Q; ++p) {
     const int i = first + 32 * p + lane;
     me[p] = i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool far = pair_far<NDIM>(me[p]);
-    const float x = far ? INFINITY : me[p].x, y = far ? INFINITY : me[p].y, z = far ? INFINITY : me[p].z;
-    MX[p] = pk2(x, x), MY[p] = pk2(y, y), MZ[p] = pk2(z, z);
+    MX[p] = pk2(me[p].x, me[p].x), MY[p] = pk2(me[p].y, me[p].y), MZ[p] = pk2(me[p].z, me[p].z);
     AX[p] = AY[p] = AZ[p] = 0;
-    if (far) close = INFINITY;
+    far_point |= pair_far<NDIM>(me[p]);
   }
+  far_point = __any_sync(FL_FULL, far_point);
   constexpr int K = 2;  // pairs of sources at a time
+  const float close = fmaxf(below(dmin2), 0.f);  // l <= close: distanceMin, or no distance at all
   float4* sa = s_a[warp];
   float4* sb = s_b[warp];
   for (int base = 32 * (rank * kPairWarps + warp); base < n; base += 32 * kPairWarps * blocks) {
     const int j = base + lane;
-    float4 o = make_float4(kPairNowhere, kPairNowhere, kPairNowhere, 0.f);
-    if (j < n) {
-      const float w = strength[j];
-      if (w != 0.f) o = pos[j], o.w = w * alpha;
-    }
-    const bool one_by_one = __any_sync(FL_FULL, pair_far<NDIM>(o));
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j < n) o = pos[j], o.w = strength[j];
+    if (o.w == 0.f) o.x = o.y = o.z = kPairNowhere;
+    o.w *= alpha;
+    const bool apart = far_point || __any_sync(FL_FULL, pair_far<NDIM>(o));
     __syncwarp();
     {
       float* pa = reinterpret_cast<float*>(&sa[lane >> 1]) + (lane & 1);
@@ -1946,6 +1946,24 @@ __global__ void __launch_bounds__(kPairThreads) k_allpairs(
       pa[0] = o.x, pa[2] = o.y, pb[0] = o.z, pb[2] = o.w;
     }
     __syncwarp();
+    // pair k of the tile, source by source
+    auto one_by_one = [&](int k, auto dmax) {
+      const float4 u = sa[k], v = sb[k];
+      const uint32_t at = (uint32_t)(base + 2 * k);
+#pragma unroll
+      for (int p = 0; p < Q; ++p) {
+        float2 ax = up2(AX[p]), ay = up2(AY[p]), az = up2(AZ[p]);
+        const uint32_t i = (uint32_t)(first + 32 * p + lane);
+        pair_term<NDIM, decltype(dmax)::value>(me[p], i, make_float4(u.x, u.z, v.x, v.z), at, dmin2, dmax2, step, seed, ax.x, ay.x, az.x);
+        pair_term<NDIM, decltype(dmax)::value>(me[p], i, make_float4(u.y, u.w, v.y, v.w), at + 1, dmin2, dmax2, step, seed, ax.y, ay.y, az.y);
+        AX[p] = pk2(ax.x, ax.y), AY[p] = pk2(ay.x, ay.y), AZ[p] = pk2(az.x, az.y);
+      }
+    };
+    if (apart) {
+#pragma unroll 1
+      for (int k = 0; k < 16; ++k) one_by_one(k, std::true_type());
+      continue;
+    }
 #pragma unroll 1
     for (int k = 0; k < 16; k += K) {
       float4 a[K], b[K];
@@ -1971,11 +1989,11 @@ __global__ void __launch_bounds__(kPairThreads) k_allpairs(
           if (NDIM > 1) cmin = fminf(fminf(cmin, fabsf(dy.x)), fabsf(dy.y));
           if (NDIM > 2) cmin = fminf(fminf(cmin, fabsf(dz.x)), fabsf(dz.y));
         }
-      bool odd = one_by_one || lmin <= close || cmin == 0.f;
+      bool odd = lmin <= close || cmin == 0.f;
       // in a small layout mostly the point itself: then as if infinitely far (in a large one it is
       // met too seldom for what the test costs in registers)
       if (Q == 1 && __any_sync(FL_FULL, odd)) {
-        odd = one_by_one;
+        odd = false;
 #pragma unroll
         for (int c = 0; c < K; ++c) {
           const int self = first + lane - (base + 2 * (k + c));
@@ -1987,19 +2005,8 @@ __global__ void __launch_bounds__(kPairThreads) k_allpairs(
         }
       }
       if (__any_sync(FL_FULL, odd)) {
-#pragma unroll
-        for (int p = 0; p < Q; ++p) {
-          float2 ax = up2(AX[p]), ay = up2(AY[p]), az = up2(AZ[p]);
-          const uint32_t i = (uint32_t)(first + 32 * p + lane);
 #pragma unroll 1
-          for (int c = 0; c < K; ++c) {
-            const float4 u = sa[k + c], v = sb[k + c];
-            const uint32_t at = (uint32_t)(base + 2 * (k + c));
-            pair_term<NDIM>(me[p], i, make_float4(u.x, u.z, v.x, v.z), at, dmin2, dmax2, step, seed, ax.x, ay.x, az.x);
-            pair_term<NDIM>(me[p], i, make_float4(u.y, u.w, v.y, v.w), at + 1, dmin2, dmax2, step, seed, ax.y, ay.y, az.y);
-          }
-          AX[p] = pk2(ax.x, ax.y), AY[p] = pk2(ay.x, ay.y), AZ[p] = pk2(az.x, az.y);
-        }
+        for (int c = 0; c < K; ++c) one_by_one(k + c, std::bool_constant<DMAX>());
         continue;
       }
 #pragma unroll
