@@ -84,7 +84,9 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 // its 128 threads 16 residues each: the block lays a tile of nodes out in shared memory, where nodes j
 // and j + 16 lie as a pair for the packed arithmetic, and a thread tests its residue's pairs, two at a
 // time (four: 22 us, eight: 26), with the very roundings of pair_push; those with an overlap go to
-// pair_push one by one. Bound by the reads of shared memory, two 16-byte loads a pair (11 us of them).
+// pair_push one by one, from the registers of the test (read again from shared memory, half as many per
+// load, 8,191 nodes that nearly all overlap took 233 us a tick, 188 so; with one scalar pair_push per
+// pair 212). Bound by the reads of shared memory, two 16-byte loads a pair (11 us of them).
 // 5,003 nodes in 2D (ncu): 45 us with one scalar pair_push per pair, now 20.
 constexpr int kPairNodes = 8, kPairResidues = 16, kPairThreads = kPairNodes * kPairResidues;
 constexpr int kPairTile = 512;  // 256 took 20.7 us, 1,024 20.3
@@ -136,9 +138,10 @@ __global__ void __launch_bounds__(kPairThreads) k_collide_allpairs(
 #pragma unroll 2
     for (int g = 0; g < kPairTile / 32; g += 2) {
       bool hit = false;
+      float4 ta[2], tb[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const float4 a = s_a[(g + k) * kPairResidues + residue], b = s_b[(g + k) * kPairResidues + residue];
+        const float4 a = ta[k] = s_a[(g + k) * kPairResidues + residue], b = tb[k] = s_b[(g + k) * kPairResidues + residue];
         const uint64_t DX = sub2(MX, pack2(a.x, a.y));
         uint64_t L;
         if (NDIM > 1) {
@@ -156,13 +159,14 @@ __global__ void __launch_bounds__(kPairThreads) k_collide_allpairs(
         hit |= l.x < r2.x || l.y < r2.y;
       }
       if (!hit || !live) continue;
-#pragma unroll 1
-      for (int k = 0; k < 4; ++k) {
-        const int at = (g + (k >> 1)) * kPairResidues + residue, j = base + (g + (k >> 1)) * 32 + (k & 1) * 16 + residue;
-        if (j >= n || j == i) continue;
-        const float* pa = reinterpret_cast<const float*>(&s_a[at]) + (k & 1);
-        const float* pb = reinterpret_cast<const float*>(&s_b[at]) + (k & 1);
-        pair_push(me, ri, make_float4(pa[0], pa[2], pb[0], pb[2]), i, nullptr, j, 0u, NDIM, strength, step, seed, acc);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int j = base + (g + k) * 32 + residue;
+        const float4 a = ta[k], b = tb[k];
+        if (j < n && j != i)
+          pair_push(me, ri, make_float4(a.x, a.z, b.x, b.z), i, nullptr, j, 0u, NDIM, strength, step, seed, acc);
+        if (j + 16 < n && j + 16 != i)
+          pair_push(me, ri, make_float4(a.y, a.w, b.y, b.w), i, nullptr, j + 16, 0u, NDIM, strength, step, seed, acc);
       }
     }
   }
