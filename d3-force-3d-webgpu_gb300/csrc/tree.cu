@@ -172,22 +172,32 @@ __device__ __forceinline__ uint64_t cell_of(float x, float origin, int e, uint32
 }
 
 // d3 cover() of a bounding box (d3-octree): origin = floor(min); a power-of-two size doubled
-// until max < origin + size (FP64). cube5 = origin x, y, z, size, log2 size, written by lane 0; every
-// lane of the warp calls it, and tries a size of its own: one thread's chain of FP64 sums and
-// compares took 3,600 clocks for 11 doublings, at the start of every tick.
-__device__ void d3_cover(const FlReduce* red, int ndim, float* cube5) {
+// until max < origin + size (FP64). cube5 = origin x, y, z, size, log2 size. WARP: every lane of the
+// warp calls it for one box, tries a size of its own, and lane 0 writes: one thread's chain of FP64 sums
+// and compares took 3,600 clocks for 11 doublings, at the start of every tick. Otherwise by one thread.
+template <bool WARP>
+__device__ __forceinline__ void d3_cover(const FlReduce* red, int ndim, float* cube5) {
   double lo0 = 0, lo1 = 0, lo2 = 0, hi0 = 0, hi1 = 0, hi2 = 0;
   lo0 = floor((double)fl::unordered(~red->lo[0])), hi0 = (double)fl::unordered(red->hi[0]);
   if (ndim > 1) lo1 = floor((double)fl::unordered(~red->lo[1])), hi1 = (double)fl::unordered(red->hi[1]);
   if (ndim > 2) lo2 = floor((double)fl::unordered(~red->lo[2])), hi2 = (double)fl::unordered(red->hi[2]);
+  const auto holds = [&](double size) {
+    return hi0 < lo0 + size && (ndim < 2 || hi1 < lo1 + size) && (ndim < 3 || hi2 < lo2 + size);
+  };
+  if (!WARP) {
+    double size = 1;
+    int lg = 0;
+    while (lg < 1100 && !holds(size)) size *= 2, ++lg;
+    cube5[0] = (float)lo0, cube5[1] = (float)lo1, cube5[2] = (float)lo2;
+    cube5[3] = (float)size, cube5[4] = (float)lg;
+    return;
+  }
   // lane k tries the size 2^(base + k); past 2^1023 doubling gives infinity
   const auto size_of = [](int k) { return k < 1024 ? __longlong_as_double((long long)(k + 1023) << 52) : (double)INFINITY; };
   int lg = 1100;
   for (int base = 0; base < 1100; base += 32) {
     const int k = base + (int)fl::lane_id();
-    const double size = size_of(k);
-    const uint32_t fits = __ballot_sync(FL_FULL, k < 1100 && hi0 < lo0 + size && (ndim < 2 || hi1 < lo1 + size) &&
-                                                     (ndim < 3 || hi2 < lo2 + size));
+    const uint32_t fits = __ballot_sync(FL_FULL, k < 1100 && holds(size_of(k)));
     if (fits) {
       lg = base + __ffs(fits) - 1;
       break;
@@ -228,7 +238,7 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const float4* __restr
   __shared__ uint32_t sh[8 * 256];
   const int passes = (64 - lo_bit + 7) / 8;
   if (threadIdx.x < 32) {
-    d3_cover(red, ndim, s_cube);
+    d3_cover<true>(red, ndim, s_cube);
     if (blockIdx.x == 0 && threadIdx.x == 0)
       for (int k = 0; k < 5; ++k) cube_out[k] = s_cube[k];
   }
@@ -255,23 +265,24 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const float4* __restr
 
 // ---- batches of graphs: the per-graph tick values, the keys, and the sort by graph
 
-// One warp per graph: the graph's d3 cube from its bounding box, the walk's threshold, its
+// One warp per graph (WARP) or one thread: the graph's d3 cube from its bounding box, the walk's threshold, its
 // distances, this tick's alpha, its velocity multiplier and its centre force's shift.
-__global__ void __launch_bounds__(kThreads) k_bgraph(int graphs, int ndim, const int32_t* __restrict__ off,
-                                                     const FlReduce* __restrict__ red,
-                                                     const FlBatchParams* __restrict__ prm,
-                                                     const double* __restrict__ alpha,
-                                                     FlGraph* __restrict__ gr) {
-  const int g = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  if (g >= graphs) return;  // the whole warp
+template <bool WARP>
+__global__ void __launch_bounds__(128) k_bgraph(int graphs, int ndim, const int32_t* __restrict__ off,
+                                        const FlReduce* __restrict__ red,
+                                        const FlBatchParams* __restrict__ prm,
+                                        const double* __restrict__ alpha,
+                                        FlGraph* __restrict__ gr) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) / (WARP ? 32 : 1);
+  if (g >= graphs) return;  // WARP: the whole warp
   FlGraph o;
   const int first = off[g], count = off[g + 1] - off[g];
   if (count > 0) {
-    d3_cover(red + g, ndim, o.origin);
+    d3_cover<WARP>(red + g, ndim, o.origin);
   } else {
     o.origin[0] = o.origin[1] = o.origin[2] = 0.f, o.size = 1.f, o.lg = 0.f;
   }
-  if (fl::lane_id()) return;
+  if (WARP && fl::lane_id()) return;
   const FlBatchParams p = prm[g];
   o.T0 = (float)((double)o.size * (double)o.size / p.theta2);
   o.dmin2 = (float)p.dmin2;
@@ -1098,7 +1109,7 @@ __global__ void __launch_bounds__(kSmallMaxThreads) k_small_tree(const SmallTree
   const uint32_t idx0 = (uint32_t)i;
   float4 p = ok ? a.pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   if (warp == 0) {
-    d3_cover(a.red, ndim, s_cube);
+    d3_cover<true>(a.red, ndim, s_cube);
     if (c == 0 && lane == 0)
       for (int k = 0; k < 5; ++k) a.cube[k] = s_cube[k];
   }
@@ -2422,7 +2433,13 @@ void fl_launch_allpairs(const float4* pos, const float* strength, float4* vel, i
 
 void fl_launch_bgraph(int graphs, int ndim, const int32_t* off, const FlReduce* red,
                       const FlBatchParams* prm, const double* alpha, FlGraph* gr, cudaStream_t st) {
-  k_bgraph<<<(graphs + 3) / 4, 128, 0, st>>>(graphs, ndim, off, red, prm, alpha, gr);
+  // A warp per graph has the shorter chain, while the FP64 pipe (2 lanes a clock) takes the warps of an SM
+  // side by side; beyond that its one active lane costs what 32 would. 512 graphs: 7.5 us with a warp each,
+  // 8.7 with a thread; 1,024: 10.1 and 8.7; 16,384: 89 and 9.4.
+  if (graphs <= 4 * fl_sms())
+    k_bgraph<true><<<(graphs + 3) / 4, 128, 0, st>>>(graphs, ndim, off, red, prm, alpha, gr);
+  else
+    k_bgraph<false><<<(graphs + 31) / 32, 32, 0, st>>>(graphs, ndim, off, red, prm, alpha, gr);
 }
 
 void fl_launch_bmorton(const float4* pos, int n, int ndim, const uint32_t* gid, const FlGraph* gr,
