@@ -1522,7 +1522,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks) k_walk(
       uint4 e = has ? sget(sp - 1 - lane) : make_uint4(0u, 0u, 0u, 0u);
       if (has && (e.x >= slot_cap || e.y - 1u >= slot_cap - e.x)) {  // a malformed tree: never read past it
         atomicOr(err, FL_ERR_TREE);
-        e.x = 0u, e.y = 1u;
+        e.x = 0u, e.y = 1u, e.w = 0u;  // a child that no point tests
       }
       const uint32_t inc = inclusive_sum(e.y), exc = inc - e.y;
       const uint32_t avail = __shfl_sync(FL_FULL, inc, 31), total = min(avail, 32u);
@@ -1762,7 +1762,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
       uint32_t ex = se.x, ey = se.y & kCountMask;
       if (has && (ex >= slot_cap || ey - 1u >= slot_cap - ex)) {  // a malformed tree: never read past it
         atomicOr(err, FL_ERR_TREE);
-        ex = 0u, ey = 1u;
+        ex = slot_cap - 1u, ey = 1u;  // the last slot: no tree fills it, and its value is 0
       }
       const uint32_t inc = inclusive_sum(ey), exc = inc - ey;
       const uint32_t avail = __shfl_sync(FL_FULL, inc, 31), total = min(avail, 32u);
