@@ -43,10 +43,10 @@ __device__ __forceinline__ float jiggle(uint32_t a, uint32_t b, uint32_t axis, u
                                         uint32_t seed) {
   uint32_t lo = a < b ? a : b, hi = a < b ? b : a;
   uint32_t h = mix32(lo ^ mix32(hi ^ mix32(seed ^ mix32(step * 4u + axis))));
-  float j = ((float)h * 2.3283064365386963e-10f - 0.5f) * 1e-6f;
-  // 193 values of h round to the middle, which would leave a pair without a displacement: there the
-  // draw is taken from the whole number, half a step off the middle
-  if (j == 0.f) j = ((float)(int32_t)(h - 0x80000000u) + 0.5f) * 2.3283064365386963e-10f * 1e-6f;
+  const float u = (float)h * 2.3283064365386963e-10f - 0.5f;
+  // 193 values of h round to the middle, which would leave a pair without a displacement: they draw
+  // 2^-33. Its bits are below those of every other draw, negative ones too: one integer maximum.
+  const float j = __uint_as_float(max(__float_as_uint(u), 0x2f000000u)) * 1e-6f;
   return a <= b ? j : -j;
 }
 
