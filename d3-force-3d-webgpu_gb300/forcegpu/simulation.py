@@ -91,6 +91,7 @@ class _NodeMirror:
         self.enqueued = 0
         self.landed = 0
         self.stale = False
+        self.again = None  # of each place, whether its node has been listed before (None: nowhere)
         self.shadow = np.zeros((0, 3))
         self.pinned = np.zeros(0, np.uint8)
         self.pinnedAt = np.zeros((0, 3))
@@ -167,6 +168,8 @@ class _NodeMirror:
         untouched = np.ones(m, bool)  # since the last exchange
         for k, axis in enumerate(axes):
             untouched &= _column(nodes, axis) == self.shadow[:m, k]
+        if self.again is not None:
+            untouched &= ~self.again[:m]
         self.shadow[:m, :self.nDim][untouched] = at[untouched]
         mine = nodes if untouched.all() else [node for node, u in zip(nodes, untouched.tolist()) if u]
         for k, axis in enumerate(axes):
@@ -179,6 +182,11 @@ class _NodeMirror:
     # --- engine calls ---
     def set_nodes(self, nodes, nDim):
         self.nodes, self.n, self.nDim = nodes, len(nodes), nDim
+        # a node object listed again lands where it came first, and is an edit at its other places
+        self.again = None
+        if len(set(map(id, nodes))) < self.n:
+            self.again = np.ones(self.n, bool)
+            self.again[np.unique([id(node) for node in nodes], return_index=True)[1]] = False
         self.enqueued = self.landed = 0
         self.plan, self.sent = [], {}
         self.upload_all(first=True)
