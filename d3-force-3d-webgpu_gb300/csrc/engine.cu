@@ -688,6 +688,13 @@ int32_t collect_errors(fl_sim* s) {
 // The message fl_last_error(NULL) returns, set by entry points that take no simulation.
 void fl_set_sim_free_error(const std::string& msg) { g_create_error = msg; }
 
+// The device bytes of a layout of n nodes with a charge and a collide force: positions, velocities, pins,
+// the link snapshot and the packed transfers (108 B a node), up to four arrays of a number per node, the
+// charge's sort and tree, the collide's sort and grid. Links (80 B each) are left to the caller's margin.
+int64_t fl_layout_bytes(int64_t n) {
+  return 124 * n + (int64_t)(2 * fl_sort_bytes(n) + fl_tree_bytes(n) + fl_grid_bytes(n));
+}
+
 extern "C" {
 
 int32_t fl_create(int32_t device, fl_sim** out) {
@@ -759,9 +766,7 @@ int32_t fl_fits(fl_sim* s, int64_t count, int32_t* fits) {
   if (!fits || count < 0) return fail(s, FL_E_ARG, "bad arguments");
   size_t freeb = 0, total = 0;
   FL_CK(s, cudaMemGetInfo(&freeb, &total));
-  // state 16 * 4 + 4 B, tree and sort ~ 200 B, per node, with a margin
-  const double need = (double)count * 300.0;
-  *fits = count <= kMaxNodes && need < 0.9 * (double)(freeb + s->pos.bytes * 8);
+  *fits = count <= kMaxNodes && (double)fl_layout_bytes(count) < 0.9 * (double)(freeb + s->pos.bytes * 8);
   return FL_OK;
 }
 

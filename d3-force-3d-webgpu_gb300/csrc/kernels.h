@@ -284,6 +284,7 @@ struct FlGridBufs {
   float4* sorted;     // [n] sorted snapshot position, radius
 };
 size_t fl_grid_bytes(int64_t n);
+int64_t fl_layout_bytes(int64_t n);  // engine.cu
 void fl_grid_carve(FlGridBufs* g, void* base, int64_t n);
 void fl_launch_grid_keys(const float4* pos, const float4* vel, int n, int ndim, float inv_cell,
                          int bits, uint64_t* keys, uint32_t* vals, uint32_t* hist, int lo_bit,
