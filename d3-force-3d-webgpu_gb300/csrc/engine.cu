@@ -292,7 +292,7 @@ int32_t ensure_scratch(fl_sim* s, Pass* p) {
   if (p->type == FL_FORCE_COLLIDE) bytes += fl_grid_bytes(n) + 256;
   FL_CK(s, p->scratch.alloc(bytes));
   // zero: the sort's counters and look-back words and the walk's group counter start at 0 (each
-  // sort and walk leaves them at 0 again)
+  // sort and walk leaves them at 0 again), and the last child slot is a child of value 0
   FL_CK(s, cudaMemset(p->scratch.p, 0, bytes));
   char* base = p->scratch.as<char>();
   fl_sort_carve(&p->sb, base, n);

@@ -189,12 +189,13 @@ struct FlTreeBufs {
   uint32_t* flag;        // [n-1] mixed-sign recursion: arrivals of each head's child cells
   float4* cell;          // [n-1] head: centroid, value at its own depth
   float4* leaf;          // [n] sorted points: position, strength
-  float4* child_data;    // [2n] slot: centroid or position, value at own depth / strength
-  uint2* child_meta;     // [2n] slot: (first child slot, count | depth << 26) or (sorted index, ~0)
-  double* slot64;        // [2n] slot of a cell: d3's FP64 value at its depth (mixed-sign recursion)
+  // [2n + 1] slots; a tree fills 2n - 1 of them, and a simulation's last one stays as allocated, zero
+  float4* child_data;    // slot: centroid or position, value at own depth / strength
+  uint2* child_meta;     // slot: (first child slot, count | depth << 26) or (sorted index, ~0)
+  double* slot64;        // slot of a cell: d3's FP64 value at its depth (mixed-sign recursion)
   void* scan_scratch;
-  double* wsum;          // [5n] per sorted point |a|, |a| x, |a| y, |a| z, a; then their prefix sums
-  double* wtiles;        // [5 tiles] partial sums of the prefix scan
+  double* wsum;          // [4n] fixed-point records of the sorted points (64-bit), prefix-summed per block
+  double* wtiles;        // [4 blocks] the blocks' totals, then their exclusive prefix
   uint32_t* omask;       // [n-1] occupied octants of each head's cell; << 16, those of its child cells
   uint32_t* head_of;     // [2n-1] d3 child: its head | octant << 27 | 1 << 31 (internal, then points)
   uint4* spill;          // the walk stacks' overflow, one region per warp slot of its grid
@@ -202,13 +203,6 @@ struct FlTreeBufs {
   int walk_slots;        // warp slots of the persistent walk grid
   int walk_blocks;       // blocks per SM of that grid (0: as many as fit)
   int sms;               // SMs of the device
-};
-struct FlWalkParams {
-  float thresh[32];   // (cube size / 2^k)^2 / theta^2
-  float damp[32];     // sqrt(4 / 2^dims)^j
-  float dmin2, dmax2;
-  int ndim;
-  uint32_t step, seed;
 };
 size_t fl_tree_bytes(int64_t n);
 // Warp slots of the persistent walk grid for n points on the current device.

@@ -334,8 +334,6 @@ __global__ void __launch_bounds__(kMortonThreads) k_bmorton(const float4* __rest
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
-// The second sort's input: the graph of each point in Morton order, in the top `passes` bytes of the
-// key, and the point's Morton-order position; with the histograms of those digits.
 // The graph of node `node`: the last g with off[g] <= node (graph offsets in shared memory).
 __device__ __forceinline__ uint32_t graph_of(const int32_t* s_off, int graphs, uint32_t node) {
   int lo = 0, hi = graphs - 1;
@@ -346,6 +344,8 @@ __device__ __forceinline__ uint32_t graph_of(const int32_t* s_off, int graphs, u
   }
   return (uint32_t)lo;
 }
+// The second sort's input: the graph of each point in Morton order, in the top `passes` bytes of the
+// key, and the point's Morton-order position; with the histograms of those digits.
 constexpr int kGidSearchMax = 8192;  // graphs whose offsets the key kernel searches in shared memory
 
 __global__ void __launch_bounds__(kMortonThreads) k_bgidkey(int n, const uint32_t* __restrict__ mperm,
@@ -545,11 +545,10 @@ __device__ __forceinline__ uint3 karras_node(const uint64_t* __restrict__ k, int
   return make_uint3((uint32_t)first, (uint32_t)last, (uint32_t)dep);
 }
 
-// The binary radix tree over the sorted keys (karras_node): thread i takes internal node i, gathers
+// The binary radix tree over the sorted keys (karras_node): thread i takes internal node i, or gathers
 // sorted point i and, for the closed-form cell sums, its record (point_record), prefix-summed within
 // the block. Integer sums are exact, and cheap where FP64 is not.
-// PART: 1, the points (sorted leaves, records, their block prefix); 2, the internal nodes;
-// 0, both in one kernel.
+// PART: 1, the points (sorted leaves, records, their block prefix); 2, the internal nodes.
 // 6 blocks per SM (40 registers): the points' half 28.1 -> 26.5 us at 1M nodes, the heads (below)
 // 30.3 -> 28.5; 8 blocks (32 registers) spill, 26.8 and 30.2.
 constexpr int kTreeBlocks = 6;
@@ -575,16 +574,16 @@ __global__ void __launch_bounds__(kThreads, kTreeBlocks) k_build(
   const uint64_t ki = i < n ? k[i] : 0;
   const int up = i < n ? kdelta(k, lo, hi, ki, i, i + 1) : -1;
   const int dn = i < n ? kdelta(k, lo, hi, ki, i, i - 1) : -1;
-  if (PART != 2 && i < n && lo == hi) leaf_parent[i] = kNoParent;  // alone in its graph: no tree
+  if (PART == 1 && i < n && lo == hi) leaf_parent[i] = kNoParent;  // alone in its graph: no tree
   D4 wrec = mk4(0, 0, 0, 0);
-  if (PART != 2 && i < n) {
+  if (PART == 1 && i < n) {
     const uint32_t node = perm[i];
     float4 p = pos[node];
     p.w = strength[node];
     leaf[i] = p;
     if (wsum) wrec = point_record(p, up, dn, ndim, cb, fe);
   }
-  if (PART != 2 && wsum)  // block-uniform
+  if (PART == 1 && wsum)  // block-uniform
     block_prefix4(wrec, wsum, wtot, i < n ? i : -1);
   if (PART == 1 || i >= n - 1) return;
   omask[i] = 0u;  // k_frontier marks the octants
@@ -813,10 +812,9 @@ __global__ void __launch_bounds__(kThreads, kTreeBlocks) k_heads(int n, int ndim
 // values, summed in FP64 above fp64_depth and in FP32 below. fp64_depth 0 runs all of it in
 // FP32 (values within 2^-20 of their children's |values| count as 0), for precision
 // comparisons.
-// Children whose slots are loaded together, and nodes per warp: with 8 and 256 the pass alone takes
-// 87 us, but 120 registers slow the tick beside others' (316 us for 312).
-constexpr int kUpBatch = 1;
 constexpr uint32_t kNoHead = 0xffffffffu;
+// Nodes per warp: 256, with eight children's slots loaded together, takes 87 us alone, but its 120
+// registers slow the tick beside others' (316 us for 312).
 constexpr int kUpThreads = 128, kUpWarps = kUpThreads / 32, kUpNodes = 128;
 
 // One head of the recursion: combine its children into its cell, write the cell into its slot
@@ -853,49 +851,32 @@ __device__ __forceinline__ uint32_t cells_up_one(
   double sv = 0, sa = 0, sx = 0, sy = 0, sz = 0;
   float fv = 0, fa = 0, fx = 0, fy = 0, fz = 0;
   float4 firstpos = make_float4(0, 0, 0, 0);
-  for (uint32_t j0 = 0; j0 < cnt; j0 += kUpBatch) {
-    uint2 m[kUpBatch];
-    float4 q[kUpBatch];
-    double v64[kUpBatch];
-#pragma unroll
-    for (int k = 0; k < kUpBatch; ++k) {
-      if (j0 + k < cnt) {
-        m[k] = cmeta[fs + j0 + k];
-        q[k] = __ldcg(cdata + fs + j0 + k);
-        v64[k] = exact ? __ldcg(slot64 + fs + j0 + k) : 0.0;
-      }
+  for (uint32_t j = 0; j < cnt; ++j) {
+    const uint2 m = cmeta[fs + j];
+    const float4 q = __ldcg(cdata + fs + j);
+    double v = exact ? __ldcg(slot64 + fs + j) : 0.0;  // a point's strength, as k_slots wrote it, or a cell's value
+    float v32 = q.w;  // the centroid weight's value
+    if (m.y != kLeafMark) {
+      // the chain of one-child cells from D + 1 down to the child's depth scales by c
+      const int cd = (int)(m.y >> 26);
+      v32 *= damp(ndim, cd - D - 1);
+      if (exact)
+        for (int l = cd - D - 1; l > 0; --l) v *= c1;
     }
-#pragma unroll
-    for (int k = 0; k < kUpBatch; ++k) {
-      if (j0 + k >= cnt) break;
-      float v32 = q[k].w;  // the centroid weight's value
-      double v = 0;
-      if (m[k].y == kLeafMark) {
-        v = v64[k];  // the point's strength, as k_slots wrote it
-      } else {
-        // the chain of one-child cells from D + 1 down to the child's depth scales by c
-        const int cd = (int)(m[k].y >> 26);
-        v32 *= damp(ndim, cd - D - 1);
-        if (exact) {
-          v = v64[k];
-          for (int l = cd - D - 1; l > 0; --l) v *= c1;
-        }
-      }
-      if (j0 + k == 0) firstpos = q[k];
-      const float a = fabsf(v32);
-      if (exact) {
-        // d3 skips children whose value is 0 (or NaN): tested on the bits
-        const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-        if (b == 0 || b > 0x7ff0000000000000ull) continue;
-        sv += v;
-      } else {
-        if (!(a > 0.f)) continue;
-        fv += v32;
-      }
-      fa += a;
-      if (wide) sa += a, sx += (double)a * q[k].x, sy += (double)a * q[k].y, sz += (double)a * q[k].z;
-      else fx += a * q[k].x, fy += a * q[k].y, fz += a * q[k].z;
+    if (j == 0) firstpos = q;
+    const float a = fabsf(v32);
+    if (exact) {
+      // d3 skips children whose value is 0 (or NaN): tested on the bits
+      const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+      if (b == 0 || b > 0x7ff0000000000000ull) continue;
+      sv += v;
+    } else {
+      if (!(a > 0.f)) continue;
+      fv += v32;
     }
+    fa += a;
+    if (wide) sa += a, sx += (double)a * q.x, sy += (double)a * q.y, sz += (double)a * q.z;
+    else fx += a * q.x, fy += a * q.y, fz += a * q.z;
   }
   float4 out;
   if (wide)
