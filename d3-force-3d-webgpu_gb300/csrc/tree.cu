@@ -467,8 +467,9 @@ __device__ __forceinline__ D4 point_record(float4 p, int up, int dn, int ndim, c
 // most its largest value then, a compare instead of a count of leading zeros.
 __device__ __forceinline__ uint64_t prefix_mask(int d) { return d < 63 ? ~0ull >> (d + 1) : 0ull; }
 // WIDE: 12 and then 7 probes at once, for a few warps an SM, which wait for each probe's latency: 5,300
-// clocks for 7,400 at 1,000 points (4 blocks of 256). With 24 warps an SM, or a chip full of them, the
-// probes' work counts and one at a time is faster (10,300 clocks for 11,600 at 5,000 points).
+// clocks for 7,400 at 1,000 points (4 blocks of 256), a tick up to 4 % shorter from 500 to 2,048. Blocks of
+// 512 show no difference; with 24 warps an SM, or a chip full of them, the probes' work counts and one at
+// a time is faster (10,300 clocks for 11,600 at 5,000 points).
 template <bool WIDE>
 __device__ __forceinline__ uint3 karras_node(const uint64_t* __restrict__ k, int lo, int hi, uint64_t ki,
                                              int up, int dn, int i, int ndim, uint32_t* left,
@@ -1028,7 +1029,7 @@ __global__ void __launch_bounds__(kThreads) k_slots(
 // The rest reads what other blocks wrote after a cluster barrier (release / acquire).
 // Bound by the chain of dependent steps, not by work: a launch, and an L2 round trip per pass. Against
 // eight launches and two memsets (the keys, a sort by counting, the tree's passes) a tick went from
-// 20.5 to 15.7 us at 1,000 points and from 44.9 to 35.2 at 5,000 (2D, with collide).
+// 20.5 to 14.3 us at 1,000 points and from 44.9 to 34.3 at 5,000 (2D, with collide).
 constexpr int kSmallRun = 256, kSmallMaxThreads = 768, kSmallBlocks = 8;
 static_assert(kSmallTreeMax == kSmallMaxThreads * kSmallBlocks, "a point per thread");
 struct SmallTree {
@@ -1858,15 +1859,17 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_lanes(
 // source. The warps' sums are added in a fixed order, in shared memory and then
 // over the cluster's.
 //
-// Bound by the FP32 pipe and instruction issue: a pair of sources takes 10 packed instructions of
-// 2 cycles each and 25 issue slots. 20,000 points in 3D: 212 us (110 is the packed instructions
-// alone), where one thread per point and sixteenth of the sources, each source tested in scalars,
-// took 757; 4,000 points 64 -> 20, 1,000 points 21 -> 10. Blocks of 128 threads: 256 wait longer
+// Bound by the FP32 pipe and instruction issue (57 % of the slots): a pair of sources and a point take
+// 10 packed instructions of 2 cycles each, 22 instructions in all. 20,000 points in 3D: 212 us alone
+// (110 is the packed instructions), where one thread per point and sixteenth of the sources, each source
+// tested in scalars, took 757; 4,000 points 64 -> 18, 1,000 points 21 -> 9. Blocks of 128 threads: 256 wait longer
 // for their slowest warp (249 us).
 constexpr int kPairThreads = 128;
 constexpr int kPairWarps = kPairThreads / 32;
 constexpr int kPairClusterMax = 8;
-constexpr int kPairTwoPoints = 10000;  // more points than this: two per lane
+// More points than this: two per lane. Ticks in 3D with one and with two: 9,000 points 62 and 65 us, 10,000
+// 73 and 72, 12,000 98 and 93 (in 2D 8,000 already take 44 and 42).
+constexpr int kPairTwoPoints = 10000;
 constexpr float kPairFar = 8.5070592e37f;  // 2^126: no difference of coordinates below it overflows
 constexpr float kPairNowhere = 1.1529215e18f;  // 2^60: finite squares, and no subnormal distance nearby
 // whether a coordinate of p is kPairFar or more, infinite or NaN
